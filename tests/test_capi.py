@@ -98,6 +98,18 @@ def test_shoup_factor_formula_host(tmp_path):
     assert out.stdout.startswith("ok")
 
 
+def test_residue_sums_equal_chain_host(tmp_path):
+    """Residue sums with an exact tail against the slot-by-slot chain: equal wherever they
+    vouch for a chain, vouching for words as queries and databases have them, and refusing
+    unreduced query words and chains that pass 2^64 (xpir_b200/csrc/residue_sum.cuh)."""
+    exe = tmp_path / "test_residue_sum"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-o", str(exe), str(ROOT / "tests" / "cpp" / "test_residue_sum.cpp"),
+                    str(ROOT / "xpir_b200" / "csrc" / "params.cpp")], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.startswith("ok")
+
+
 def test_admission_and_continuous_batching_host(tmp_path):
     """The serving loop's queueing rules (xpir_b200/csrc/admission.h) under a fake executor:
     FIFO per lane, budget never exceeded, oversize refused, batches formed from arrivals,

@@ -80,7 +80,7 @@ Sizes sizes_of(const xpir_b200_ctx *ctx, const std::vector<Group> &groups) {
   Sizes z;
   for (const Group &g : groups) {
     const uint64_t k = g.reqs.size();
-    z.tasks += k * g.d;
+    z.tasks += 2 * k * g.d;  // a level may be two launches (launch_sum_level)
     for (uint32_t lvl = 0; lvl + 1 < g.d; lvl++) {
       z.ws_a = std::max<size_t>(z.ws_a, k * g.sh.groups[lvl] * g.sh.P[lvl] * ct_bytes);
       z.ws_b = std::max<size_t>(z.ws_b, k * g.sh.groups[lvl] * g.sh.P[lvl + 1] * mN * 8);
@@ -89,9 +89,11 @@ Sizes sizes_of(const xpir_b200_ctx *ctx, const std::vector<Group> &groups) {
   return z;
 }
 
-// Enqueues every launch of the batch on the context's stream.
+// Enqueues every launch of the batch on the context's stream; by_slot: every level with the
+// slot-by-slot kernel (after the residue sums asked for it).
 cudaError_t enqueue(xpir_b200_ctx *ctx, const std::vector<Group> &groups, const xpir_b200_request *reqs,
-                    uint64_t *ws_a, uint64_t *ws_b, ReplyTask *host_tasks, ReplyTask *dev_tasks) {
+                    uint64_t *ws_a, uint64_t *ws_b, ReplyTask *host_tasks, ReplyTask *dev_tasks,
+                    bool by_slot = false) {
   const uint64_t mN = (uint64_t)ctx->ps.m * ctx->ps.N, ct_words = 2 * mN, ct_bytes = ct_words * 8;
   size_t task_off = 0;
   for (const Group &g : groups) {
@@ -101,7 +103,8 @@ cudaError_t enqueue(xpir_b200_ctx *ctx, const std::vector<Group> &groups, const 
     const uint32_t k = (uint32_t)g.reqs.size();
     std::vector<const uint64_t *> db(k), q(k);
     std::vector<uint64_t *> out(k);
-    uint64_t q_off = 0;
+    uint64_t q_off = 0, live = g.sh.n_real0;  // elements past `live`: import of zero bits
+    const bool slots = by_slot || g.db->zero_polys();
     for (uint32_t lvl = 0; lvl < g.d; lvl++) {
       const bool last = lvl + 1 == g.d;
       const uint64_t P = g.sh.P[lvl], groups_l = g.sh.groups[lvl];
@@ -113,22 +116,31 @@ cudaError_t enqueue(xpir_b200_ctx *ctx, const std::vector<Group> &groups, const 
         out[i] = last ? (uint64_t *)r.replies : ws_a + (uint64_t)i * groups_l * P * ct_words;
       }
       uint32_t launched = 0;
-      cudaError_t e = launch_reply_tasks(db.data(), q.data(), out.data(), k, n_real, P, groups_l, g.n[lvl], ps, dm,
-                                         host_tasks + task_off, dev_tasks + task_off, ctx->stream, &launched,
-                                         ctx->status_dev, tuned_tile(ctx, P, g.n[lvl], groups_l), last);
+      const bool sums = !slots && sum_level(ctx, ps, n_real, live, P, g.n[lvl], groups_l, k);
+      const uint64_t active = active_groups(sums ? live : n_real, g.n[lvl], groups_l);
+      cudaError_t e =
+          sums ? launch_sum_level(sum_args(ctx, n_real, live, P, groups_l, g.n[lvl], last), db.data(), q.data(),
+                                  out.data(), k, ps, dm, host_tasks + task_off, dev_tasks + task_off, ctx->stream,
+                                  &launched)
+               : launch_reply_tasks(db.data(), q.data(), out.data(), k, n_real, P, groups_l, g.n[lvl], ps, dm,
+                                    host_tasks + task_off, dev_tasks + task_off, ctx->stream, &launched,
+                                    ctx->status_dev, tuned_tile(ctx, P, g.n[lvl], groups_l), last);
       ctx->launches += launched;
       if (e != cudaSuccess) {
         fprintf(stderr, "xpir_b200: batched reply launch failed: %s (level %u of %u, P %llu, n_i %u, groups %llu, %u tasks)\n",
                 cudaGetErrorName(e), lvl, g.d, (unsigned long long)P, g.n[lvl], (unsigned long long)groups_l, k);
         return e;
       }
-      task_off += k;
+      task_off += 2 * k;
       q_off += (uint64_t)g.n[lvl] * ct_words;
       if (last) break;
       // All queries' level replies are one run of k*groups elements of P ciphertexts; in
       // each query's row, groups past `active` replied exactly zero (and were not written).
       const AggSource as{(const uint8_t *)ws_a, (uint64_t)k * groups_l, P * ct_bytes, P * ct_bytes, 1};
-      const ImportRows rows{k, groups_l, active_groups(n_real, g.n[lvl], groups_l)};
+      ImportRows rows{k, groups_l, active};
+      rows.fill = slots || !sum_level(ctx, ps, groups_l, active, g.sh.P[lvl + 1], g.n[lvl + 1],
+                                       g.sh.groups[lvl + 1], k);
+      live = active;
       launched = 0;
       e = launch_import(as, (uint64_t)k * groups_l, g.sh.P[lvl + 1], ps, dm, ctx->d_tables, ws_b, ctx->stream,
                         &rows, &launched);
@@ -232,11 +244,22 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   }
   if (groups.empty()) return overall;
   const Sizes z = sizes_of(ctx, groups);
-  *ctx->status_host = 0;
+  ctx->status_host[0] = ctx->status_host[1] = 0;
 
-  auto finish = [&](cudaError_t err) -> int {
-    const cudaError_t se = cudaStreamSynchronize(ctx->stream);  // also on error: nothing left in flight
+  // Ends the call.  Where residue sums asked for it, the batch first runs once more slot by
+  // slot, in the given workspaces and task tables.
+  auto finish = [&](cudaError_t err, void *wa = nullptr, void *wb = nullptr, void *ht = nullptr,
+                    void *dt = nullptr) -> int {
+    cudaError_t se = cudaStreamSynchronize(ctx->stream);  // also on error: nothing left in flight
     if (err == cudaSuccess) err = se;
+    if (err == cudaSuccess && ((volatile int *)ctx->status_host)[1] != 0) {
+      ctx->status_host[0] = ctx->status_host[1] = 0;
+      err = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
+      if (err == cudaSuccess)
+        err = enqueue(ctx, groups, reqs, (uint64_t *)wa, (uint64_t *)wb, (ReplyTask *)ht, (ReplyTask *)dt, true);
+      se = cudaStreamSynchronize(ctx->stream);
+      if (err == cudaSuccess) err = se;
+    }
     if (err != cudaSuccess) ctx->last_error = err;
     int rc = status_of(err);
     if (rc == XPIR_B200_OK && *(volatile int *)ctx->status_host != 0) rc = XPIR_B200_ERR_TIMEOUT;
@@ -288,7 +311,7 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
     // with a stream synchronisation, so its copy has completed.
     e = enqueue(ctx, groups, reqs, (uint64_t *)wa, (uint64_t *)wb, (ReplyTask *)ctx->tasks_host,
                 (ReplyTask *)ctx->tasks_dev);
-    return finish(e);
+    return finish(e, wa, wb, ctx->tasks_host, ctx->tasks_dev);
   }
 
   // Graph path: replay a captured plan for the same request list, or capture one.
@@ -296,15 +319,18 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   for (auto &pl : ctx->plans)
     if (pl->key == key) {
       ctx->launches += pl->launches;
-      return finish(cudaGraphLaunch(pl->exec, ctx->stream));
+      e = cudaGraphLaunch(pl->exec, ctx->stream);
+      return finish(e, pl->ws_a, pl->ws_b, (ReplyTask *)pl->host_tasks + z.tasks, (ReplyTask *)pl->dev_tasks + z.tasks);
     }
   auto plan = std::make_shared<BatchPlan>();
   plan->key = key;
   for (const Group &g : groups) plan->db_ids.push_back(g.db->id);
   e = cudaMalloc(&plan->ws_a, std::max<size_t>(z.ws_a, 256));
   if (e == cudaSuccess) e = cudaMalloc(&plan->ws_b, std::max<size_t>(z.ws_b, 256));
-  if (e == cudaSuccess) e = cudaMalloc(&plan->dev_tasks, z.tasks * sizeof(ReplyTask));
-  if (e == cudaSuccess) e = cudaMallocHost(&plan->host_tasks, z.tasks * sizeof(ReplyTask));
+  // Two tables: the graph copies the first from host_tasks at every replay, so a repeat of the
+  // batch slot by slot fills the second.
+  if (e == cudaSuccess) e = cudaMalloc(&plan->dev_tasks, 2 * z.tasks * sizeof(ReplyTask));
+  if (e == cudaSuccess) e = cudaMallocHost(&plan->host_tasks, 2 * z.tasks * sizeof(ReplyTask));
   // One eager run first: it sets the kernels' attributes outside the capture and
   // produces this submission's replies.
   if (e == cudaSuccess)
@@ -325,7 +351,8 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   if (e != cudaSuccess) return finish(e);
   if (ctx->plans.size() >= kMaxPlans) ctx->plans.erase(ctx->plans.begin());
   ctx->plans.push_back(plan);
-  return finish(cudaSuccess);
+  return finish(cudaSuccess, plan->ws_a, plan->ws_b, (ReplyTask *)plan->host_tasks + z.tasks,
+                (ReplyTask *)plan->dev_tasks + z.tasks);
 }
 
 extern "C" int xpir_b200_reply_batch(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t count, int use_graph) {
@@ -379,7 +406,34 @@ extern "C" int xpir_b200_autotune(xpir_b200_ctx *ctx, const xpir_b200_db *db, ui
       }
     }
     if (e != cudaSuccess) break;
-    ctx->tuned[std::make_tuple(sh.P[lvl], (uint64_t)n[lvl], sh.groups[lvl])] = best;
+    // The residue sums, where they apply, against the fastest tile: a level that they reply
+    // faster stays without a pinned tile.
+    const auto level_key = std::make_tuple(sh.P[lvl], (uint64_t)n[lvl], sh.groups[lvl]);
+    ctx->tuned.erase(level_key);
+    bool sums = !db->zero_polys() && sum_level(ctx, ps, in_real, in_real, sh.P[lvl], n[lvl], sh.groups[lvl], 1);
+    if (sums) {
+      float ms = 0;
+      ReplyTask tasks[2];
+      for (int rep_i = 0; rep_i < 2 && e == cudaSuccess; rep_i++) {
+        ctx->status_host[1] = 0;
+        e = cudaEventRecord(e0, ctx->stream);
+        if (e == cudaSuccess)
+          e = launch_sum_level(sum_args(ctx, in_real, in_real, sh.P[lvl], sh.groups[lvl], n[lvl], true), &in, &q, &rep,
+                               1, ps, dm, tasks, nullptr, ctx->stream, nullptr);
+        if (e == cudaSuccess) e = cudaEventRecord(e1, ctx->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+      }
+      if (e == cudaSuccess && ((volatile int *)ctx->status_host)[1] != 0) {
+        sums = false;  // not decided by sums: the level's replies from a tile again
+        e = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
+        if (e == cudaSuccess) e = launch_reply_level(a, ps, dm, ctx->stream, nullptr, ctx->status_dev, best);
+      }
+      ctx->status_host[1] = 0;
+      if (e != cudaSuccess) break;
+      sums = sums && ms < best_ms;
+    }
+    if (!sums) ctx->tuned[level_key] = best;
     if (lvl == 0 && tile0) *tile0 = best;
     q += (uint64_t)n[lvl] * ct_words;
     if (lvl + 1 == d) break;

@@ -62,6 +62,21 @@ ParamSet with_bits(const ParamSet &base, uint32_t b) {
   return ps;
 }
 
+// Every engine kernel and the no-allocation scratch on `device` (the current one); once per
+// device, since a module stays loaded.
+cudaError_t load_kernels(int device) {
+  static std::mutex mu;
+  static std::set<int> loaded;
+  std::lock_guard<std::mutex> lock(mu);
+  if (loaded.count(device)) return cudaSuccess;
+  cudaError_t e = preload_import_kernels();
+  if (e == cudaSuccess) e = preload_reply_kernels();
+  if (e == cudaSuccess) e = preload_sum_kernels();
+  if (e == cudaSuccess) e = prepare_noalloc_scratch(device);
+  if (e == cudaSuccess) loaded.insert(device);
+  return e;
+}
+
 }  // namespace
 
 void xpir::note_cuda_error(cudaError_t e) {
@@ -137,9 +152,7 @@ int xpir_b200_ctx_create(xpir_b200_ctx **out, int device, uint32_t N, uint32_t m
   int rc = cuda_status(cudaSetDevice(device));
   // Load every engine kernel and place the no-allocation scratch on this device now, so
   // that no later call loads a module (module loading reserves device memory).
-  if (rc == XPIR_B200_OK) rc = cuda_status(preload_import_kernels());
-  if (rc == XPIR_B200_OK) rc = cuda_status(preload_reply_kernels());
-  if (rc == XPIR_B200_OK) rc = cuda_status(prepare_noalloc_scratch(device));
+  if (rc == XPIR_B200_OK) rc = cuda_status(load_kernels(device));
   if (rc == XPIR_B200_OK) rc = cuda_status(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   if (rc == XPIR_B200_OK) rc = cuda_status(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
   if (rc == XPIR_B200_OK) rc = cuda_status(cudaEventCreateWithFlags(&ctx->query_copied, cudaEventDisableTiming));
@@ -154,13 +167,27 @@ int xpir_b200_ctx_create(xpir_b200_ctx **out, int device, uint32_t N, uint32_t m
     uint64_t keep = UINT64_MAX;
     rc = cuda_status(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
   }
-  if (rc == XPIR_B200_OK) rc = cuda_status(cudaMalloc(&ctx->d_tables, tables.size() * sizeof(uint64_t)));
+  // One allocation: the tables, the zero bit stream's import and the runs' workspace.
+  const uint64_t zero_words = (uint64_t)m * N;
+  if (rc == XPIR_B200_OK)
+    rc = cuda_status(cudaMalloc(&ctx->d_tables, (tables.size() + zero_words + kPartWords + 2) * sizeof(uint64_t)));
   if (rc == XPIR_B200_OK)
     rc = cuda_status(cudaMemcpy(ctx->d_tables, tables.data(), tables.size() * sizeof(uint64_t),
                                 cudaMemcpyHostToDevice));
-  if (rc == XPIR_B200_OK) rc = cuda_status(cudaHostAlloc(&ctx->status_host, sizeof(int), cudaHostAllocMapped));
   if (rc == XPIR_B200_OK) {
-    *ctx->status_host = 0;
+    ctx->zero_poly = ctx->d_tables + tables.size();
+    ctx->ws_part = ctx->zero_poly + zero_words;
+    ctx->stop_flag = (int *)(ctx->ws_part + kPartWords);
+    rc = cuda_status(cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream));
+  }
+  if (rc == XPIR_B200_OK) {
+    rc = cuda_status(launch_zero_poly(ctx->ps, make_dev_moduli(ctx->ps), ctx->d_tables, ctx->zero_poly, ctx->stream));
+  }
+  if (rc == XPIR_B200_OK) rc = cuda_status(cudaHostAlloc(&ctx->status_host, (2 + kZeroHints) * sizeof(int),
+                                                         cudaHostAllocMapped));
+  if (rc == XPIR_B200_OK) {
+    ctx->status_host[0] = ctx->status_host[1] = 0;
+    for (int i = 1 + kZeroHints; i >= 2; i--) ctx->free_hints.push_back(i);
     rc = cuda_status(cudaHostGetDevicePointer((void **)&ctx->status_dev, ctx->status_host, 0));
   }
   if (rc != XPIR_B200_OK) {
@@ -286,7 +313,7 @@ int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, uint64_t nb_el
   db->b = b;
   db->alpha = alpha;
   db->element_bytes = element_bytes;
-  cudaError_t e = cudaMalloc(&db->d_polys, words * sizeof(uint64_t));
+  cudaError_t e = cudaMalloc(&db->d_polys, (words + 2) * sizeof(uint64_t));  // the last two: zero_seen
   if (e != cudaSuccess) {
     delete db;
     return cuda_status(e);
@@ -299,8 +326,17 @@ int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, uint64_t nb_el
     src = (const uint8_t *)staging;
   }
   if (e == cudaSuccess) {
-    const AggSource as{src, nb_elements, element_bytes, element_stride, alpha};
-    e = launch_import(as, groups, P, ps, make_dev_moduli(ps), ctx->d_tables, db->d_polys, ctx->stream);
+    AggSource as{src, nb_elements, element_bytes, element_stride, alpha};
+    if (!ctx->free_hints.empty()) {
+      db->hint = ctx->free_hints.back();
+      ctx->free_hints.pop_back();
+      ctx->status_host[db->hint] = 0;
+      as.zero_seen = (int *)(db->d_polys + words);
+      as.zero_hint = ctx->status_dev + db->hint;
+      e = cudaMemsetAsync(as.zero_seen, 0, sizeof(int), ctx->stream);
+    }
+    if (e == cudaSuccess)
+      e = launch_import(as, groups, P, ps, make_dev_moduli(ps), ctx->d_tables, db->d_polys, ctx->stream);
     ctx->launches++;
   }
   if (staging) {
@@ -310,6 +346,7 @@ int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, uint64_t nb_el
   }
   if (e != cudaSuccess) {
     cudaFree(db->d_polys);
+    if (db->hint) ctx->free_hints.push_back(db->hint);
     delete db;
     return cuda_status(e);
   }
@@ -327,6 +364,7 @@ int xpir_b200_db_free(xpir_b200_db *db) {
   cudaStreamSynchronize(ctx->stream);
   drop_plans_of(ctx, db->id);
   cudaFree(db->d_polys);
+  if (db->hint) ctx->free_hints.push_back(db->hint);
   delete db;
   return XPIR_B200_OK;
 }
@@ -420,9 +458,6 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
     dq = (const uint64_t *)ctx->ws_query;
   }
 
-  const uint64_t *in = db->d_polys;
-  uint64_t in_real = db->n_agg;
-  *ctx->status_host = 0;
   // Event pairs of this call (kernel timing): [2*lvl] the level's reply, [2*lvl+1] the
   // re-import after it; a pair is read only when its launch was recorded.
   bool timed[2 * XPIR_B200_MAX_LEVELS] = {};
@@ -434,41 +469,65 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
     timed[k] = true;
     return cudaEventRecord(ctx->timing_ev[k][1], ctx->stream);
   };
-  for (uint32_t lvl = 0; lvl < d; lvl++) {
-    const bool last = lvl + 1 == d;
-    uint64_t *rep = (last && out_on_device) ? (uint64_t *)replies : (uint64_t *)ctx->ws_a;
-    uint32_t launched = 0;
-    if (lvl == 1 && split_copy) XPIR_TRY(cudaStreamWaitEvent(ctx->stream, ctx->query_copied, 0));
-    ReplyLevelArgs a{in, in_real, Ps[lvl], groups[lvl], n[lvl], dq, rep};
-    a.write_idle = last;
-    a.wait_test = ctx->wait_test;
-    const uint64_t active = active_groups(in_real, n[lvl], groups[lvl]);
-    XPIR_TRY(time_begin(2 * lvl));
-    const cudaError_t le = launch_reply_level(a, ps, dm, ctx->stream, &launched, ctx->status_dev,
-                                              tuned_tile(ctx, Ps[lvl], n[lvl], groups[lvl]));
-    if (le == cudaErrorNotSupported) return XPIR_B200_ERR_ARG;
-    XPIR_TRY(le);
-    XPIR_TRY(time_end(2 * lvl, launched));
-    ctx->launches += launched;
-    dq += (uint64_t)n[lvl] * ct_words;
-    if (last) break;
-    // Level replies -> next level's database: element e's Ps[lvl] ciphertexts are one
-    // contiguous bit stream (no inverse NTT, as the reference).
-    // Groups past `active` replied exactly zero (and were not written out).
-    const AggSource as{(const uint8_t *)rep, groups[lvl], Ps[lvl] * ct_bytes, Ps[lvl] * ct_bytes, 1};
-    const ImportRows rows{1, groups[lvl], active};
-    launched = 0;
-    XPIR_TRY(time_begin(2 * lvl + 1));
-    XPIR_TRY(launch_import(as, groups[lvl], Ps[lvl + 1], ps, dm, ctx->d_tables, (uint64_t *)ctx->ws_b,
-                           ctx->stream, &rows, &launched));
-    XPIR_TRY(time_end(2 * lvl + 1, launched));
-    ctx->launches += launched;
-    in = (const uint64_t *)ctx->ws_b;
-    in_real = groups[lvl];
+  // Every level's launches and the copy of the replies; by_slot: all levels slot by slot.
+  auto run_levels = [&](bool by_slot) -> int {
+    const uint64_t *in = db->d_polys, *q = dq;
+    uint64_t in_real = db->n_agg, in_live = db->n_agg;  // elements past in_live: import of zero bits
+    ctx->status_host[0] = ctx->status_host[1] = 0;
+    for (uint32_t lvl = 0; lvl < d; lvl++) {
+      const bool last = lvl + 1 == d;
+      uint64_t *rep = (last && out_on_device) ? (uint64_t *)replies : (uint64_t *)ctx->ws_a;
+      uint32_t launched = 0;
+      if (lvl == 1 && split_copy) XPIR_TRY(cudaStreamWaitEvent(ctx->stream, ctx->query_copied, 0));
+      const bool sums = !by_slot && sum_level(ctx, ps, in_real, in_live, Ps[lvl], n[lvl], groups[lvl], 1);
+      const uint64_t active = active_groups(sums ? in_live : in_real, n[lvl], groups[lvl]);
+      XPIR_TRY(time_begin(2 * lvl));
+      cudaError_t le;
+      if (sums) {
+        ReplyTask tasks[2];
+        le = launch_sum_level(sum_args(ctx, in_real, in_live, Ps[lvl], groups[lvl], n[lvl], last), &in, &q, &rep, 1, ps,
+                              dm, tasks, nullptr, ctx->stream, &launched);
+      } else {
+        ReplyLevelArgs a{in, in_real, Ps[lvl], groups[lvl], n[lvl], q, rep};
+        a.write_idle = last;
+        a.wait_test = ctx->wait_test;
+        le = launch_reply_level(a, ps, dm, ctx->stream, &launched, ctx->status_dev,
+                                tuned_tile(ctx, Ps[lvl], n[lvl], groups[lvl]));
+      }
+      if (le == cudaErrorNotSupported) return XPIR_B200_ERR_ARG;
+      XPIR_TRY(le);
+      XPIR_TRY(time_end(2 * lvl, launched));
+      ctx->launches += launched;
+      q += (uint64_t)n[lvl] * ct_words;
+      if (last) break;
+      // Level replies -> next level's database: element e's Ps[lvl] ciphertexts are one
+      // contiguous bit stream (no inverse NTT, as the reference).
+      // Groups past `active` replied exactly zero (and were not written out); residue sums
+      // do not read their import.
+      const AggSource as{(const uint8_t *)rep, groups[lvl], Ps[lvl] * ct_bytes, Ps[lvl] * ct_bytes, 1};
+      ImportRows rows{1, groups[lvl], active};
+      rows.fill = by_slot || !sum_level(ctx, ps, groups[lvl], active, Ps[lvl + 1], n[lvl + 1],
+                                         groups[lvl + 1], 1);
+      launched = 0;
+      XPIR_TRY(time_begin(2 * lvl + 1));
+      XPIR_TRY(launch_import(as, groups[lvl], Ps[lvl + 1], ps, dm, ctx->d_tables, (uint64_t *)ctx->ws_b,
+                             ctx->stream, &rows, &launched));
+      XPIR_TRY(time_end(2 * lvl + 1, launched));
+      ctx->launches += launched;
+      in = (const uint64_t *)ctx->ws_b;
+      in_real = groups[lvl];
+      in_live = active;
+    }
+    if (!out_on_device)
+      XPIR_TRY(cudaMemcpyAsync(replies, ctx->ws_a, final_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    XPIR_TRY(cudaStreamSynchronize(ctx->stream));
+    return XPIR_B200_OK;
+  };
+  if ((rc = run_levels(db->zero_polys())) != XPIR_B200_OK) return rc;
+  if (((volatile int *)ctx->status_host)[1] != 0) {
+    XPIR_TRY(cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream));
+    if ((rc = run_levels(true)) != XPIR_B200_OK) return rc;
   }
-  if (!out_on_device)
-    XPIR_TRY(cudaMemcpyAsync(replies, ctx->ws_a, final_bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  XPIR_TRY(cudaStreamSynchronize(ctx->stream));
   for (uint32_t k = 0; k < 2 * d; k++) {
     if (!timed[k]) continue;
     float ms = 0;

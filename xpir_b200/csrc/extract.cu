@@ -29,6 +29,7 @@
 #include "modarith.cuh"
 #include "ntt.cuh"
 #include "params.h"
+#include "residue_sum.cuh"
 #include "xpir_b200.h"
 
 namespace xpir {
@@ -45,22 +46,9 @@ struct LiftConsts {
   uint64_t inv_shoup[kMaxLiftModuli];  // floor(inv * 2^64 / p_c)
 };
 
-// Exact reductions modulo one of XPIR's moduli (2^60 < p < 2^61 with D = 2^61 - p below
-// 2^23 for all 17 of them), which give the unique residue the reference's GMP lift
-// computes.  A 64-bit word w: q0 = w >> 61 <= 7 and w - q0*p = (w mod 2^61) + q0*D lies
-// in [0, 2p) whenever 9*D < 2^61.
-__device__ __forceinline__ uint64_t mod_word(uint64_t w, uint64_t p, uint64_t np) {
-  const uint64_t r = w + (w >> 61) * np;
-  return r >= p ? r - p : r;
-}
-
-// h*2^64 + l mod p for h < p: h*2^64 mod p = h*2^64 - f*p with f = floor(h*2^64/p) (the
-// Shoup factor of h), whose low word is f*(2^64 - p).
-__device__ __forceinline__ uint64_t mod_two_words(uint64_t h, uint64_t l, uint64_t p, uint64_t np, uint32_t delta) {
-  const uint64_t s = shoup_factor8_np(h, p, np, delta) * np + mod_word(l, p, np);  // < 2p
-  return s >= p ? s - p : s;
-}
-
+// Exact reductions modulo one of XPIR's moduli (mod_word, mod_two_words) give the unique
+// residue the reference's GMP lift computes.
+//
 // x (its low nl of kLimbs little-endian limbs) mod p, from the top limb down; the loop is
 // unrolled over all limbs so that x stays in registers.
 __device__ __forceinline__ uint64_t limbs_mod_fast(const uint64_t (&x)[kLimbs], int nl, uint64_t p, uint64_t np,

@@ -31,7 +31,7 @@ struct xpir_b200_ctx {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t query_copied = nullptr;
   xpir::ParamSet ps;           // b is set per database
-  uint64_t *d_tables = nullptr;
+  uint64_t *d_tables = nullptr;  // also holds zero_poly and ws_part
   std::mutex mu;
   std::atomic<uint64_t> launches{0};  // engine kernels launched (also counted off the lock)
   std::atomic<int> servers{0};         // servers with a lane on this context
@@ -50,8 +50,14 @@ struct xpir_b200_ctx {
   // generation, extraction): it keeps freed memory for the next call (release threshold
   // UINT64_MAX), so that a call after the first maps no new device memory.
   cudaMemPool_t pool = nullptr;
-  int *status_host = nullptr;  // kernel status word (mapped pinned memory)
+  // mapped pinned memory: [0] kernel status, [1] redo (SumLevelArgs), then kZeroHints ints
+  // that databases hold one of each (xpir_b200_db::hint)
+  int *status_host = nullptr;
   int *status_dev = nullptr;
+  uint64_t *zero_poly = nullptr;  // [m][N]: import of a zero bit stream
+  int *stop_flag = nullptr;       // SumLevelArgs::stop
+  uint64_t *ws_part = nullptr;    // residues of runs (SumLevelArgs::part), kPartWords words
+  std::vector<int> free_hints;   // indexes of status_host that no database holds
   std::set<xpir_b200_db *> dbs;  // databases imported through this context
   TuneTable tuned;
   uint64_t tune_epoch = 0;  // bumped by every autotune (invalidates captured batches)
@@ -64,6 +70,13 @@ struct xpir_b200_ctx {
   uint64_t reply_timed[XPIR_B200_MAX_LEVELS] = {}, import_timed = 0;
   std::vector<std::shared_ptr<BatchPlan>> plans;  // captured batches (batch.cu)
 };
+
+constexpr int kZeroHints = 1022;
+
+// Workspace of the residue sums' runs: 1.8 MiB per context, made with it, so that no reply
+// allocates it (a level takes as many runs as fit; the 100,000 x 4 KB level's 27 take 221,184
+// words).
+constexpr uint64_t kPartWords = 240000;
 
 // Tile shape for a level shape: the autotuned one if any, else -1 (default).
 inline int tuned_tile(const xpir_b200_ctx *ctx, uint64_t P, uint64_t n_i, uint64_t groups) {
@@ -80,7 +93,26 @@ struct xpir_b200_db {
   uint32_t b = 0;
   uint32_t alpha = 1;
   uint64_t element_bytes = 0;
+  // Index in status_host of this database's zero hint (AggSource), 0: none.  Words 0 and p,
+  // the import of zero bits, keep the residue sums from deciding a chain, so replies from a
+  // database with all-zero polys run slot by slot at once.  Only a hint: it may be set late
+  // (imports from device memory are asynchronous), and the sums notice by themselves.
+  int hint = 0;
+  bool zero_polys() const { return hint && ((volatile int *)ctx->status_host)[hint] != 0; }
 };
+
+// Whether a level takes the residue-sum path: no pinned or tuned tile shape, no wait test.
+inline bool sum_level(const xpir_b200_ctx *ctx, const xpir::ParamSet &ps, uint64_t n_real, uint64_t n_live, uint64_t P,
+                      uint64_t n_i, uint64_t groups, uint64_t ntasks) {
+  return ctx->wait_test.spin_limit == 0 && ctx->wait_test.withhold_tile < 0 &&
+         tuned_tile(ctx, P, n_i, groups) < 0 && xpir::sum_level_supported(ps, n_real, n_live, P, n_i, groups, ntasks);
+}
+
+inline xpir::SumLevelArgs sum_args(const xpir_b200_ctx *ctx, uint64_t n_real, uint64_t n_live, uint64_t P,
+                                   uint64_t n_groups, uint64_t n_i, bool write_idle) {
+  return {n_real,       n_live,     P, n_groups, n_i, write_idle, ctx->zero_poly, ctx->ws_part, kPartWords,
+          ctx->status_dev + 1, ctx->status_dev, ctx->stop_flag};
+}
 
 struct xpir_b200_request;
 

@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kImportMaxThreads) import_kernel(const AggSour
   const bool flat = (real == src.alpha) && (src.alpha == 1 || src.element_stride == src.element_bytes);
   const uint8_t *flat_base = src.base + first * src.element_stride;
   const bool aligned = flat && ((((uintptr_t)flat_base) & 7) == 0);
+  uint64_t any = 0;
   for (uint32_t w = threadIdx.x; w < sh.stage_words; w += blockDim.x) {
     const uint64_t bpos = byte0 + 8ull * w;
     uint64_t v = 0;
@@ -116,8 +117,10 @@ __global__ void __launch_bounds__(kImportMaxThreads) import_kernel(const AggSour
       }
     }
     stage[w] = v;
+    any |= v;
   }
-  __syncthreads();
+  if (!__syncthreads_or(any != 0) && threadIdx.x == 0 && c == 0 && src.zero_seen && atomicExch(src.zero_seen, 1) == 0)
+    *(volatile int *)src.zero_hint = 1;
 
   // Coefficient k, twisted by phi^k: b <= 56 one chunk per coefficient; b > 56 sub-chunks
   // of 56 bits combined per modulus as sum_t mulmod(s_t, 2^(56t)) without a final
@@ -215,7 +218,7 @@ cudaError_t launch_import(const AggSource &src, uint64_t groups, uint64_t P, con
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (launches) (*launches)++;
   }
-  if (zero_polys > 0) {
+  if (zero_polys > 0 && r.fill) {
     const size_t zsmem = (size_t)ps.N * sizeof(uint64_t);
     cudaError_t e = allow_max_dynamic_smem((const void *)import_zero_fill_kernel);
     if (e != cudaSuccess) return e;
@@ -230,6 +233,21 @@ cudaError_t launch_import(const AggSource &src, uint64_t groups, uint64_t P, con
     if (launches) (*launches)++;
   }
   return cudaSuccess;
+}
+
+cudaError_t launch_zero_poly(const ParamSet &ps, const DevModuli &dm, const uint64_t *tables, uint64_t *out,
+                             cudaStream_t stream) {
+  ImportShape sh{};
+  sh.N = ps.N;
+  sh.log_n = ps.log_n;
+  sh.m = ps.m;
+  sh.P = 1;
+  sh.per_row = 1;  // one element, known zero
+  cudaError_t e = allow_max_dynamic_smem((const void *)import_zero_fill_kernel);
+  if (e != cudaSuccess) return e;
+  import_zero_fill_kernel<<<dim3(1, ps.m), import_threads(ps.N), (size_t)ps.N * sizeof(uint64_t), stream>>>(sh, dm, tables,
+                                                                                                      out, 1);
+  return cudaGetLastError();
 }
 
 // Loads both import kernels on the current device (lazy module loading would otherwise do

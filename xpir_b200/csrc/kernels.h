@@ -22,6 +22,10 @@ struct AggSource {
   uint64_t element_bytes;
   uint64_t element_stride;
   uint32_t alpha;
+  // Optional: *zero_seen (device memory, cleared by the caller) and *zero_hint (host memory)
+  // are set when the bits of some poly, and those next to them, are all zero.
+  int *zero_seen = nullptr;
+  int *zero_hint = nullptr;
 };
 
 // Per-modulus constants the device needs, by value.
@@ -49,7 +53,12 @@ DevModuli make_dev_moduli(const ParamSet &ps);
 // by the kernels launched.
 struct ImportRows {
   uint64_t rows, per_row, active;
+  bool fill = true;  // false: the known-zero elements are left unwritten (nobody reads them)
 };
+
+// The constant import of an all-zero bit stream, one poly per modulus: out[m][N].
+cudaError_t launch_zero_poly(const ParamSet &ps, const DevModuli &dm, const uint64_t *tables, uint64_t *out,
+                             cudaStream_t stream);
 
 // The secret key's Shoup factors (sks = floor(sk * 2^64 / p), sk words below p) for
 // query generation and extraction, computed on the device on `stream`.
@@ -108,6 +117,7 @@ struct alignas(128) ReplyTask {
   CUtensorMap tm_db;
   CUtensorMap tm_q;
   uint64_t *out;
+  const uint64_t *db, *query;  // the maps' bases (read by the residue-sum kernels only)
 };
 
 // A compiled tile shape of the reply kernel: W coefficients per slice, C columns per
@@ -147,10 +157,35 @@ inline uint64_t active_groups(uint64_t n_real, uint64_t n_i, uint64_t n_groups) 
 // path, degree a multiple of 16, 32-bit TMA coordinates).
 bool reply_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_i, uint64_t groups);
 
+// One recursion level by residue sums and an exact tail (reply_sum.cu), for `ntasks` queries
+// of the same shape: db[t], query[t], out[t] as in ReplyLevelArgs.  Of the n_real elements
+// only the first n_live are in db; the rest are the constant import of a zero bit stream
+// (zero_poly) and their replies, exactly zero, are written only with write_idle.  A level
+// whose replies cannot be shown to equal the slot-by-slot kernel's sets *redo (a
+// device-visible int that the caller clears): the caller then repeats the call with that
+// kernel.
+struct SumLevelArgs {
+  uint64_t n_real, n_live, P, n_groups, n_i;
+  bool write_idle;
+  const uint64_t *zero_poly;
+  uint64_t *part;       // workspace of part_words words
+  uint64_t part_words;
+  int *redo, *status;
+  int *stop;  // device memory: set with *redo, cleared by the caller before it repeats the call
+};
+// Whether a level of this shape takes that path.
+bool sum_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_live, uint64_t P, uint64_t n_i,
+                         uint64_t groups, uint64_t ntasks);
+// host_tasks (and dev_tasks, when ntasks > 1): 2 * ntasks entries.
+cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, const uint64_t *const *query,
+                             uint64_t *const *out, uint32_t ntasks, const ParamSet &ps, const DevModuli &dm,
+                             ReplyTask *host_tasks, ReplyTask *dev_tasks, cudaStream_t stream, uint32_t *launches);
+
 // Load the import and reply kernels on the current device, so that no later launch
 // loads a module (which reserves device memory).
 cudaError_t preload_import_kernels();
 cudaError_t preload_reply_kernels();
+cudaError_t preload_sum_kernels();
 // Places the scratch array of xpir_b200_reply_noalloc on the current device (loading
 // the module that holds it) and caches its device address (noalloc.cu).
 cudaError_t prepare_noalloc_scratch(int device);

@@ -134,37 +134,56 @@ extern "C" int xpir_b200_reply_noalloc(xpir_b200_ctx *ctx, const xpir_b200_db *d
   if (e == cudaSuccess && d > 1) e = scratch_address(ctx->device, &scratch);
   if (e != cudaSuccess) return status_of(e);
 
-  *ctx->status_host = 0;
-  const uint64_t *in = db->d_polys;
-  const uint64_t *q = (const uint64_t *)query_dev;
-  uint64_t in_real = db->n_agg;
-  for (uint32_t lvl = 0; lvl < d; lvl++) {
-    const bool last = lvl + 1 == d;
-    uint64_t *rep = last ? (uint64_t *)replies_dev : (uint64_t *)scratch;
-    uint32_t launched = 0;
-    // As xpir_b200_reply: intermediate levels leave the replies of groups without data
-    // unwritten, and the next import fills those groups with their constant poly.
-    ReplyLevelArgs a{in, in_real, Ps[lvl], groups[lvl], n[lvl], q, rep};
-    a.write_idle = last;
-    const uint64_t active = active_groups(in_real, n[lvl], groups[lvl]);
-    e = launch_reply_level(a, ps, dm, ctx->stream, &launched, ctx->status_dev,
-                           tuned_tile(ctx, Ps[lvl], n[lvl], groups[lvl]));
-    ctx->launches += launched;
+  // Every level's launches; by_slot: all levels slot by slot (as xpir_b200_reply).
+  auto run_levels = [&](bool by_slot) -> cudaError_t {
+    const uint64_t *in = db->d_polys;
+    const uint64_t *q = (const uint64_t *)query_dev;
+    uint64_t in_real = db->n_agg, in_live = db->n_agg;
+    ctx->status_host[0] = ctx->status_host[1] = 0;
+    for (uint32_t lvl = 0; lvl < d; lvl++) {
+      const bool last = lvl + 1 == d;
+      uint64_t *rep = last ? (uint64_t *)replies_dev : (uint64_t *)scratch;
+      uint32_t launched = 0;
+      const bool sums = !by_slot && sum_level(ctx, ps, in_real, in_live, Ps[lvl], n[lvl], groups[lvl], 1);
+      // Intermediate levels leave the replies of groups without data unwritten; the next
+      // import fills those groups with their constant poly where the next level reads it.
+      const uint64_t active = active_groups(sums ? in_live : in_real, n[lvl], groups[lvl]);
+      cudaError_t le;
+      if (sums) {
+        ReplyTask tasks[2];
+        le = launch_sum_level(sum_args(ctx, in_real, in_live, Ps[lvl], groups[lvl], n[lvl], last), &in, &q, &rep, 1, ps,
+                              dm, tasks, nullptr, ctx->stream, &launched);
+      } else {
+        ReplyLevelArgs a{in, in_real, Ps[lvl], groups[lvl], n[lvl], q, rep};
+        a.write_idle = last;
+        le = launch_reply_level(a, ps, dm, ctx->stream, &launched, ctx->status_dev,
+                                tuned_tile(ctx, Ps[lvl], n[lvl], groups[lvl]));
+      }
+      ctx->launches += launched;
+      if (le != cudaSuccess) return le;
+      q += (uint64_t)n[lvl] * ct_words;
+      if (last) break;
+      uint64_t *next = (uint64_t *)(scratch + off_b);
+      const AggSource as{(const uint8_t *)rep, groups[lvl], Ps[lvl] * ct_bytes, Ps[lvl] * ct_bytes, 1};
+      ImportRows rows{1, groups[lvl], active};
+      rows.fill = by_slot || !sum_level(ctx, ps, groups[lvl], active, Ps[lvl + 1], n[lvl + 1],
+                                         groups[lvl + 1], 1);
+      launched = 0;
+      le = launch_import(as, groups[lvl], Ps[lvl + 1], ps, dm, ctx->d_tables, next, ctx->stream, &rows, &launched);
+      ctx->launches += launched;
+      if (le != cudaSuccess) return le;
+      in = next;
+      in_real = groups[lvl];
+      in_live = active;
+    }
+    return cudaStreamSynchronize(ctx->stream);
+  };
+  if ((e = run_levels(db->zero_polys())) != cudaSuccess) return status_of(e);
+  if (((volatile int *)ctx->status_host)[1] != 0) {
+    e = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess) e = run_levels(true);
     if (e != cudaSuccess) return status_of(e);
-    q += (uint64_t)n[lvl] * ct_words;
-    if (last) break;
-    uint64_t *next = (uint64_t *)(scratch + off_b);
-    const AggSource as{(const uint8_t *)rep, groups[lvl], Ps[lvl] * ct_bytes, Ps[lvl] * ct_bytes, 1};
-    const ImportRows rows{1, groups[lvl], active};
-    launched = 0;
-    e = launch_import(as, groups[lvl], Ps[lvl + 1], ps, dm, ctx->d_tables, next, ctx->stream, &rows, &launched);
-    ctx->launches += launched;
-    if (e != cudaSuccess) return status_of(e);
-    in = next;
-    in_real = groups[lvl];
   }
-  e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) return status_of(e);
   if (*(volatile int *)ctx->status_host != 0) return XPIR_B200_ERR_TIMEOUT;
   if (nb_replies) *nb_replies = final_count;
   return XPIR_B200_OK;
