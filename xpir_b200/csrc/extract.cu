@@ -62,19 +62,19 @@ __device__ __forceinline__ uint64_t limbs_mod_fast(const uint64_t (&x)[kLimbs], 
   return r;
 }
 
+template <int LOGN>
 __global__ void __launch_bounds__(256, 4) decrypt_poly_kernel(const uint64_t *__restrict__ ct,
-                                                           const uint64_t *__restrict__ sk,
-                                                           const uint64_t *__restrict__ sks,
-                                                           const uint64_t *__restrict__ tables, uint32_t N,
-                                                           uint32_t log_n, uint32_t m, const DevModuli dm,
-                                                           uint64_t *__restrict__ res) {
-  extern __shared__ uint64_t poly[];
+                                                              const uint64_t *__restrict__ sk,
+                                                              const uint64_t *__restrict__ sks,
+                                                              const uint64_t *__restrict__ tables, uint32_t m,
+                                                              const DevModuli dm, uint64_t *__restrict__ res) {
+  constexpr uint32_t N = 1u << LOGN, shift = 32 - LOGN;
+  extern __shared__ __align__(16) uint64_t poly[];
   const uint32_t c = blockIdx.y;
   const uint64_t j = blockIdx.x;
   const uint64_t p = dm.p[c];
   const uint64_t *a = ct + (j * 2 * m + c) * N, *b = ct + (j * 2 * m + m + c) * N;
   const uint64_t *s = sk + (uint64_t)c * N, *ss = sks + (uint64_t)c * N;
-  const uint32_t shift = 32 - log_n;
 #pragma unroll 4
   for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {  // unrolled: several rows of loads in flight
     const uint64_t temp = shoup_mac(0, a[i], s[i], ss[i], p);  // in [0, p)
@@ -85,14 +85,16 @@ __global__ void __launch_bounds__(256, 4) decrypt_poly_kernel(const uint64_t *__
   }
   __syncthreads();
   const uint64_t *tab = tables + (uint64_t)c * kTableSlots * N;
-  ntt_lazy_rb<3>(poly, tab + kInvOmega * N, tab + kInvOmegaShoup * N, N, log_n, p,
-                 [&](uint32_t k) { return poly[swz(k)]; });
-  const uint64_t *iphi = tab + kInvPhi * N, *iphis = tab + kInvPhiShoup * N;
+  ntt_lazy<LOGN, false, true>(poly, reinterpret_cast<const ulonglong2 *>(tab + kInvOmega * N), p,
+                              [&](uint32_t k) { return poly[swz(k)]; });
+  const ulonglong2 *iphi = reinterpret_cast<const ulonglong2 *>(tab + kInvPhi * N);
   uint64_t *o = res + (j * m + c) * N;
   // In output order (coalesced global loads and stores); the bit reversal is its own
   // inverse, so output k reads transform slot brev(k).
-  for (uint32_t k = threadIdx.x; k < N; k += blockDim.x)
-    o[k] = shoup_mul(poly[swz(__brev(k) >> shift)], iphi[k], iphis[k], p);
+  for (uint32_t k = threadIdx.x; k < N; k += blockDim.x) {
+    const ulonglong2 f = __ldg(iphi + k);
+    o[k] = shoup_mul(poly[swz(__brev(k) >> shift)], f.x, f.y, p);
+  }
 }
 
 __global__ void __launch_bounds__(256) lift_pack_kernel(const uint64_t *__restrict__ res, uint64_t nct, uint32_t N,
@@ -258,7 +260,6 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
       e = cudaMemcpyAsync(d_in, replies, top * ct_words * 8, cudaMemcpyHostToDevice, st);
     level_in = d_in;
   }
-  if (e == cudaSuccess) e = allow_max_dynamic_smem((const void *)decrypt_poly_kernel);
   for (uint32_t lvl = d; lvl >= 1 && e == cudaSuccess; lvl--) {
     const uint64_t nbr = extract_count(aggregated_bytes, lvl, bits, N, m);
     uint64_t *res = nullptr, *out = nullptr;
@@ -271,9 +272,16 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
     if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, out_words * 8, st);
     if (e == cudaSuccess && nbr > 0x7fffffffull) e = cudaErrorInvalidValue;
     if (e == cudaSuccess) {
-      decrypt_poly_kernel<<<dim3((unsigned)nbr, m), 256, N * 8, st>>>(level_in, d_sk, d_sks, ctx->d_tables, N,
-                                                                    ps.log_n, m, dm, res);
-      e = cudaGetLastError();
+#define XPIR_DECRYPT(L)                                                                                           \
+  {                                                                                                               \
+    e = allow_max_dynamic_smem((const void *)decrypt_poly_kernel<L>);                                             \
+    if (e == cudaSuccess) {                                                                                       \
+      decrypt_poly_kernel<L><<<dim3((unsigned)nbr, m), 256, N * 8, st>>>(level_in, d_sk, d_sks, ctx->d_tables, m, \
+                                                                        dm, res);                                \
+      e = cudaGetLastError();                                                                                     \
+    }                                                                                                             \
+  }
+      XPIR_BY_DEGREE(ps.log_n, XPIR_DECRYPT)
     }
     if (e == cudaSuccess) {
       const uint64_t threads = nbr * N;

@@ -33,18 +33,13 @@ DevModuli make_dev_moduli(const ParamSet &ps) {
 
 namespace {
 
-// Threads per import CTA: N/16, two 8-coefficient groups of the register-blocked NTT
-// per thread and pass (on B200 this beat one group per thread, 16-coefficient groups,
-// and the transform fed straight from the bit extraction, all bit-identical).
-constexpr uint32_t kImportMaxThreads = kMaxPolyDegree / 16;
-inline uint32_t import_threads(uint32_t N) { return N / 16; }
-
 struct ImportShape {
-  uint32_t N, log_n, m, b, nsub;
-  uint64_t P;
-  uint64_t per_row, active;  // element s of CTA u = blockIdx.x / P: (u / active) * per_row + u % active
+  uint32_t N, m, b, nsub;
+  uint32_t P, active;    // element s of CTA poly (u, j): (u / active) * per_row + u % active
+  uint64_t per_row;
+  uint64_t polys;        // polys to import: rows * active * P
   uint64_t total_bytes;  // bytes of one aggregated element (alpha * element_bytes)
-  uint32_t stage_words;  // u64 words of staged input per poly
+  uint32_t stage_words;  // u64 words of staged input per poly (even)
 };
 
 // Byte i of aggregated element s, following the reference's reused import buffer: a
@@ -69,51 +64,60 @@ __device__ __forceinline__ uint8_t agg_byte(const AggSource &src, uint64_t s, ui
 }
 
 
-// nbits (<= 56) bits starting at bit `pos` of the staged little-endian words.
-__device__ __forceinline__ uint64_t staged_bits(const uint64_t *st, uint64_t pos, uint32_t nbits) {
-  const uint64_t w = pos >> 6;
-  const uint32_t sh = (uint32_t)(pos & 63);
-  uint64_t v = st[w] >> sh;
-  if (sh) v |= st[w + 1] << (64 - sh);
-  return v & ((1ull << nbits) - 1);
+// Bits pos .. of the staged little-endian words, cut by the masks of the two result halves.
+__device__ __forceinline__ uint64_t staged_bits(const uint32_t *st, uint32_t pos, uint32_t mask_lo, uint32_t mask_hi) {
+  const uint32_t *w = st + (pos >> 5);
+  const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
+  return (uint64_t)(__funnelshift_r(w1, w2, pos) & mask_hi) << 32 | (__funnelshift_r(w0, w1, pos) & mask_lo);
+}
+__device__ __forceinline__ uint32_t low_mask(int bits) { return bits >= 32 ? ~0u : bits <= 0 ? 0u : (1u << bits) - 1; }
+
+// Eight bytes of a contiguous element from byte `at` on; bytes past `bytes` are zero.
+__device__ __forceinline__ uint64_t flat_word(const uint8_t *base, uint64_t at, uint64_t bytes) {
+  const uint8_t *p = base + at;
+  const uint32_t off = (uint32_t)(uintptr_t)p & 7;
+  const uint64_t *w = (const uint64_t *)(p - off);
+  if (off == 0 && at + 8 <= bytes) return w[0];
+  // Between two aligned words that both lie in the element.
+  if (off && at >= off && at - off + 16 <= bytes) return w[0] >> (8 * off) | w[1] << (64 - 8 * off);
+  uint64_t v = 0;
+  for (uint32_t q = 0; q < 8; q++)
+    if (at + q < bytes) v |= (uint64_t)p[q] << (8 * q);
+  return v;
 }
 
-// grid: x = aggregated element * P + poly, y = modulus; import_threads(N) threads.
-// Dynamic smem: stage words, then N words.
-__global__ void __launch_bounds__(kImportMaxThreads) import_kernel(const AggSource src, const ImportShape sh,
-                                                                   const DevModuli dm,
-                                                                   const uint64_t *__restrict__ tables,
-                                                                   uint64_t *__restrict__ out) {
+// One CTA imports one poly of one modulus: grid: x = poly, y = modulus; T threads.  ALIAS: one group of coefficients per thread
+// (T = N/8), so that the transform's buffer can take the place of the staged input once
+// every thread holds its coefficients.  Dynamic smem: the staged words and the polys.
+template <int LOGN, int T, bool ALIAS, int MINB>
+__global__ void __launch_bounds__(T, MINB) import_kernel(const AggSource src, const ImportShape sh, const DevModuli dm,
+                                                         const uint64_t *__restrict__ tables,
+                                                         uint64_t *__restrict__ out) {
+  constexpr uint32_t N = 1u << LOGN;
+  static_assert(!ALIAS || T == (int)N / 8, "aliasing needs one group per thread");
   extern __shared__ __align__(16) uint64_t smem[];
   uint64_t *stage = smem;
-  uint64_t *poly = smem + sh.stage_words;
-  const uint64_t u = blockIdx.x / sh.P, j = blockIdx.x - u * sh.P;
-  const uint64_t row = u / sh.active, s = row * sh.per_row + (u - row * sh.active);
+  uint64_t *poly = ALIAS ? smem : smem + sh.stage_words;
   const uint32_t c = blockIdx.y;
-  const uint32_t N = sh.N;
   const uint64_t p = dm.p[c];
-
+  const uint32_t u = blockIdx.x / sh.P, j = blockIdx.x - u * sh.P, row = u / sh.active;
+  const uint64_t s = row * sh.per_row + (u - row * sh.active);
   // Stage the bytes of this poly's bit range, from an 8-byte aligned start.
-  const uint64_t bit0 = j * (uint64_t)N * sh.b;
-  const uint64_t byte0 = (bit0 >> 3) & ~7ull;
+  const uint64_t bit0 = (uint64_t)j * N * sh.b, byte0 = (bit0 >> 3) & ~7ull;
   const uint64_t first = s * src.alpha;
   const uint64_t real = (first + src.alpha <= src.nb_elements) ? src.alpha : src.nb_elements - first;
   const bool flat = (real == src.alpha) && (src.alpha == 1 || src.element_stride == src.element_bytes);
-  const uint8_t *flat_base = src.base + first * src.element_stride;
-  const bool aligned = flat && ((((uintptr_t)flat_base) & 7) == 0);
+  const uint8_t *base = src.base + first * src.element_stride;
   uint64_t any = 0;
-  for (uint32_t w = threadIdx.x; w < sh.stage_words; w += blockDim.x) {
-    const uint64_t bpos = byte0 + 8ull * w;
+  for (uint32_t w = threadIdx.x; w < sh.stage_words; w += T) {
+    const uint64_t at = byte0 + 8ull * w;
     uint64_t v = 0;
-    if (bpos + 8 <= sh.total_bytes && aligned) {
-      v = *reinterpret_cast<const uint64_t *>(flat_base + bpos);
-    } else {
-      for (uint32_t q = 0; q < 8; q++) {
-        const uint64_t i = bpos + q;
-        if (i < sh.total_bytes) {
-          const uint8_t byte = flat ? flat_base[i] : agg_byte(src, s, i, real);
-          v |= (uint64_t)byte << (8 * q);
-        }
+    if (at < sh.total_bytes) {
+      if (flat) {
+        v = flat_word(base, at, sh.total_bytes);
+      } else {
+        for (uint32_t k = 0; k < 8; k++)
+          if (at + k < sh.total_bytes) v |= (uint64_t)agg_byte(src, s, at + k, real) << (8 * k);
       }
     }
     stage[w] = v;
@@ -123,33 +127,30 @@ __global__ void __launch_bounds__(kImportMaxThreads) import_kernel(const AggSour
     *(volatile int *)src.zero_hint = 1;
 
   // Coefficient k, twisted by phi^k: b <= 56 one chunk per coefficient; b > 56 sub-chunks
-  // of 56 bits combined per modulus as sum_t mulmod(s_t, 2^(56t)) without a final
-  // reduction.
+  // of 56 bits combined per modulus as sum_t mulmod(s_t, 2^(56t)) without a final reduction
+  // (the first is below p and stays as it is).
   const uint64_t *tab = tables + (uint64_t)c * kTableSlots * N;
-  const uint64_t *phi = tab + kPhi * N, *phi_s = tab + kPhiShoup * N;
-  const uint64_t rel0 = bit0 - 8 * byte0;
-  for (uint32_t k = threadIdx.x; k < N; k += blockDim.x) {
-    const uint64_t pos = rel0 + (uint64_t)k * sh.b;
-    uint64_t x;
-    if (sh.nsub == 1) {
-      x = staged_bits(stage, pos, sh.b);
-    } else {
-      x = 0;
-      for (uint32_t t = 0; t < sh.nsub; t++) {
-        const uint32_t sz = (t + 1 < sh.nsub) ? 56 : sh.b - 56 * (sh.nsub - 1);
-        const uint64_t sub = staged_bits(stage, pos + 56ull * t, sz);
-        x += shoup_mul(sub, dm.crt[c][t], dm.crt_shoup[c][t], p);
-      }
+  const ulonglong2 *phi = reinterpret_cast<const ulonglong2 *>(tab + kPhi * N);
+  const uint32_t *st = reinterpret_cast<const uint32_t *>(stage);
+  const uint32_t b = sh.b, nsub = sh.nsub, rel0 = (uint32_t)(bit0 - 8 * byte0);
+  const int first_bits = nsub == 1 ? (int)b : 56, last_bits = (int)b - 56 * (int)(nsub - 1);
+  const uint32_t mask_lo = low_mask(first_bits), mask_hi = low_mask(first_bits - 32);
+  auto coefficient = [&](uint32_t k) -> uint64_t {
+    const ulonglong2 f = __ldg(phi + k);
+    const uint32_t pos = rel0 + k * b;
+    uint64_t x = staged_bits(st, pos, mask_lo, mask_hi);
+    for (uint32_t t = 1; t < nsub; t++) {
+      const int bits = t + 1 < nsub ? 56 : last_bits;
+      x += shoup_mul(staged_bits(st, pos + 56 * t, low_mask(bits), low_mask(bits - 32)), dm.crt[c][t],
+                     dm.crt_shoup[c][t], p);
     }
-    poly[swz(k)] = shoup_mul(x, __ldg(phi + k), __ldg(phi_s + k), p);
-  }
-  __syncthreads();
-  ntt_lazy_rb<3>(poly, tab + kOmega * N, tab + kOmegaShoup * N, N, sh.log_n, p,
-                 [&](uint32_t k) { return poly[swz(k)]; });
+    return shoup_mul(x, f.x, f.y, p);
+  };
+  ntt_lazy<LOGN, ALIAS>(poly, reinterpret_cast<const ulonglong2 *>(tab + kOmega * N), p, coefficient);
 
   // Coalesced 16-byte stores; swz(2t+1) == swz(2t) ^ 1.
   ulonglong2 *o = reinterpret_cast<ulonglong2 *>(out + ((s * sh.P + j) * sh.m + c) * (uint64_t)N);
-  for (uint32_t t = threadIdx.x; t < N / 2; t += blockDim.x) {
+  for (uint32_t t = threadIdx.x; t < N / 2; t += T) {
     const uint32_t at = swz(2 * t);
     o[t] = make_ulonglong2(poly[at], poly[at ^ 1]);
   }
@@ -160,18 +161,21 @@ __global__ void __launch_bounds__(kImportMaxThreads) import_kernel(const AggSour
 // 0 and p).  Each CTA computes it for modulus blockIdx.y in shared memory, then writes it
 // to its share of the `count` known-zero polys t (element row * per_row + active +
 // (t / P) % (per_row - active) of row t / (P * (per_row - active)), poly t % P).
-__global__ void __launch_bounds__(kImportMaxThreads) import_zero_fill_kernel(const ImportShape sh,
-                                                                             const DevModuli dm,
-                                                                             const uint64_t *__restrict__ tables,
-                                                                             uint64_t *__restrict__ out,
-                                                                             uint64_t count) {
+template <int LOGN>
+__global__ void __launch_bounds__(512) import_zero_fill_kernel(const ImportShape sh, const DevModuli dm,
+                                                               const uint64_t *__restrict__ tables,
+                                                               uint64_t *__restrict__ out, uint64_t count) {
+  constexpr uint32_t N = 1u << LOGN;
   extern __shared__ __align__(16) uint64_t smem[];
-  const uint32_t c = blockIdx.y, N = sh.N;
+  const uint32_t c = blockIdx.y;
   const uint64_t p = dm.p[c];
   const uint64_t *tab = tables + (uint64_t)c * kTableSlots * N;
-  const uint64_t *phi = tab + kPhi * N, *phi_s = tab + kPhiShoup * N;
-  auto coefficient = [&](uint32_t k) -> uint64_t { return shoup_mul(0, __ldg(phi + k), __ldg(phi_s + k), p); };
-  ntt_lazy_rb<3>(smem, tab + kOmega * N, tab + kOmegaShoup * N, N, sh.log_n, p, coefficient);
+  const ulonglong2 *phi = reinterpret_cast<const ulonglong2 *>(tab + kPhi * N);
+  auto coefficient = [&](uint32_t k) -> uint64_t {
+    const ulonglong2 f = __ldg(phi + k);
+    return shoup_mul(0, f.x, f.y, p);
+  };
+  ntt_lazy<LOGN, false>(smem, reinterpret_cast<const ulonglong2 *>(tab + kOmega * N), p, coefficient);
   const uint64_t zeros = sh.per_row - sh.active;
   for (uint64_t t = blockIdx.x; t < count; t += gridDim.x) {
     const uint64_t u = t / sh.P, j = t - u * sh.P;
@@ -184,6 +188,46 @@ __global__ void __launch_bounds__(kImportMaxThreads) import_zero_fill_kernel(con
   }
 }
 
+template <int LOGN, int T, bool ALIAS, int MINB>
+cudaError_t launch_import_n(const AggSource &src, const ImportShape &sh, const DevModuli &dm, const uint64_t *tables,
+                            uint64_t *out, cudaStream_t stream) {
+  auto kern = import_kernel<LOGN, T, ALIAS, MINB>;
+  const cudaError_t e = allow_max_dynamic_smem((const void *)kern);
+  if (e != cudaSuccess) return e;
+  const size_t words = ALIAS ? std::max(sh.stage_words, sh.N) : sh.stage_words + sh.N;
+  kern<<<dim3((unsigned)sh.polys, sh.m), T, words * 8, stream>>>(src, sh, dm, tables, out);
+  return cudaGetLastError();
+}
+
+typedef cudaError_t (*ImportFn)(const AggSource &, const ImportShape &, const DevModuli &, const uint64_t *, uint64_t *,
+                                cudaStream_t);
+struct ImportEntry {
+  ImportFn import;
+  const void *kernels[2];
+};
+#define XPIR_IMPORT(LOGN, T, ALIAS, MINB)                                                       \
+  {                                                                                             \
+    &launch_import_n<LOGN, T, ALIAS, MINB>, {                                                   \
+      (const void *)import_kernel<LOGN, T, ALIAS, MINB>, (const void *)import_zero_fill_kernel<LOGN> \
+    }                                                                                           \
+  }
+// By degree 512..8192; 64 registers and 32 warps per SM (16,000 polys of 2048: 348 us, with 80
+// registers and 24 warps 369).  At 8192 a thread has two groups of coefficients.
+const ImportEntry kImports[] = {
+    XPIR_IMPORT(9, 64, true, 16),  XPIR_IMPORT(10, 128, true, 8),   XPIR_IMPORT(11, 256, true, 4),
+    XPIR_IMPORT(12, 512, true, 2), XPIR_IMPORT(13, 512, false, 2),
+};
+
+template <int LOGN>
+cudaError_t launch_zero_fill(const ImportShape &sh, const DevModuli &dm, const uint64_t *tables, uint64_t *out,
+                             uint64_t count, unsigned blocks, cudaStream_t stream) {
+  auto kern = import_zero_fill_kernel<LOGN>;
+  const cudaError_t e = allow_max_dynamic_smem((const void *)kern);
+  if (e != cudaSuccess) return e;
+  kern<<<dim3(blocks, sh.m), ntt_threads(sh.N), (size_t)sh.N * 8, stream>>>(sh, dm, tables, out, count);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_import(const AggSource &src, uint64_t groups, uint64_t P, const ParamSet &ps,
@@ -193,43 +237,37 @@ cudaError_t launch_import(const AggSource &src, uint64_t groups, uint64_t P, con
   const ImportRows r = rows ? *rows : ImportRows{1, groups, groups};
   if (r.rows == 0 || r.per_row == 0 || r.rows * r.per_row != groups || r.active > r.per_row)
     return cudaErrorInvalidValue;
+  const uint64_t computed = r.rows * r.active, zero_polys = r.rows * (r.per_row - r.active) * P;
+  if (computed * P > 0x7fffffffull || P > 0x7fffffffull) return cudaErrorInvalidValue;
   ImportShape sh;
   sh.N = ps.N;
-  sh.log_n = ps.log_n;
   sh.m = ps.m;
   sh.b = ps.b;
   sh.nsub = (ps.b + 55) / 56;
-  sh.P = P;
+  sh.P = (uint32_t)P;
   sh.per_row = r.per_row;
-  sh.active = r.active;
+  sh.active = (uint32_t)r.active;
+  sh.polys = computed * P;
   sh.total_bytes = (uint64_t)src.alpha * src.element_bytes;
-  // bits of one poly plus the in-word offset, rounded up, plus one spare word for the
-  // two-word reads of staged_bits
-  sh.stage_words = (uint32_t)((64 + (uint64_t)ps.N * ps.b + 63) / 64 + 2);
-  const size_t smem = (size_t)(sh.stage_words + ps.N) * sizeof(uint64_t);
-  const unsigned threads = import_threads(ps.N);
-  const uint64_t computed = r.rows * r.active, zero_polys = r.rows * (r.per_row - r.active) * P;
-  if (computed * P > 0x7fffffffull) return cudaErrorInvalidValue;
+  // bits of one poly plus the in-word offset, rounded up, plus spare words for the
+  // three-half-word reads of staged_bits; even, so that the polys stay 16-byte aligned
+  sh.stage_words = (uint32_t)(((64 + (uint64_t)ps.N * ps.b + 63) / 64 + 3) & ~1ull);
   if (computed > 0) {
-    cudaError_t e = allow_max_dynamic_smem((const void *)import_kernel);
+    const cudaError_t e = kImports[ps.log_n - 9].import(src, sh, dm, tables, out, stream);
     if (e != cudaSuccess) return e;
-    dim3 grid((unsigned)(computed * P), ps.m);
-    import_kernel<<<grid, threads, smem, stream>>>(src, sh, dm, tables, out);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (launches) (*launches)++;
   }
   if (zero_polys > 0 && r.fill) {
-    const size_t zsmem = (size_t)ps.N * sizeof(uint64_t);
-    cudaError_t e = allow_max_dynamic_smem((const void *)import_zero_fill_kernel);
-    if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
     // About four CTAs per SM over all moduli: each computes the constant poly once.
     const uint64_t per_mod = std::max<uint64_t>(1, 4ull * (uint64_t)sms / ps.m);
-    dim3 grid((unsigned)std::min<uint64_t>(zero_polys, per_mod), ps.m);
-    import_zero_fill_kernel<<<grid, threads, zsmem, stream>>>(sh, dm, tables, out, zero_polys);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)std::min<uint64_t>(zero_polys, per_mod);
+#define XPIR_FILL(L) e = launch_zero_fill<L>(sh, dm, tables, out, zero_polys, blocks, stream)
+    XPIR_BY_DEGREE(ps.log_n, XPIR_FILL)
+    if (e != cudaSuccess) return e;
     if (launches) (*launches)++;
   }
   return cudaSuccess;
@@ -239,24 +277,25 @@ cudaError_t launch_zero_poly(const ParamSet &ps, const DevModuli &dm, const uint
                              cudaStream_t stream) {
   ImportShape sh{};
   sh.N = ps.N;
-  sh.log_n = ps.log_n;
   sh.m = ps.m;
   sh.P = 1;
   sh.per_row = 1;  // one element, known zero
-  cudaError_t e = allow_max_dynamic_smem((const void *)import_zero_fill_kernel);
-  if (e != cudaSuccess) return e;
-  import_zero_fill_kernel<<<dim3(1, ps.m), import_threads(ps.N), (size_t)ps.N * sizeof(uint64_t), stream>>>(sh, dm, tables,
-                                                                                                      out, 1);
-  return cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+#define XPIR_ZERO(L) e = launch_zero_fill<L>(sh, dm, tables, out, 1, 1, stream)
+  XPIR_BY_DEGREE(ps.log_n, XPIR_ZERO)
+  return e;
 }
 
-// Loads both import kernels on the current device (lazy module loading would otherwise do
+// Loads the import kernels on the current device (lazy module loading would otherwise do
 // it, and reserve their device memory, at their first launch).
 cudaError_t preload_import_kernels() {
   cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, import_kernel);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, import_zero_fill_kernel);
-  return e;
+  for (const ImportEntry &entry : kImports)
+    for (const void *k : entry.kernels) {
+      const cudaError_t e = cudaFuncGetAttributes(&fa, k);
+      if (e != cudaSuccess) return e;
+    }
+  return cudaSuccess;
 }
 
 }  // namespace xpir

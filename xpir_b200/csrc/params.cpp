@@ -41,21 +41,25 @@ uint32_t ilog2(uint64_t x) {
   return r;
 }
 
+// Entry i of a table of pairs.
+void put(uint64_t *tab, uint32_t i, uint64_t v, uint64_t p) {
+  tab[2 * i] = v;
+  tab[2 * i + 1] = shoup_of(v, p);
+}
+
 // Powers of w for each butterfly layer of the lazy DIF NTT: N/2 powers of w, then N/4
-// powers of w^2, ..., one power of w^(N/2): N-1 words, the N-th left zero.
-void layer_powers(uint64_t *tab, uint64_t *tab_shoup, uint64_t w, uint32_t N, uint64_t p) {
+// powers of w^2, ..., one power of w^(N/2): N-1 entries, the N-th left zero.
+void layer_powers(uint64_t *tab, uint64_t w, uint32_t N, uint64_t p) {
   uint32_t o = 0;
   for (uint32_t K = N; K >= 2; K >>= 1) {
     uint64_t wi = 1;
     for (uint32_t i = 0; i < K / 2; i++, o++) {
-      tab[o] = wi;
-      tab_shoup[o] = shoup_of(wi, p);
+      put(tab, o, wi, p);
       wi = mulmod(wi, w, p);
     }
     w = mulmod(w, w, p);
   }
-  tab[N - 1] = 0;
-  tab_shoup[N - 1] = 0;
+  put(tab, N - 1, 0, p);
 }
 
 }  // namespace
@@ -107,26 +111,23 @@ bool build_params(uint32_t N, uint32_t m, uint32_t b, ParamSet *ps, std::vector<
       t = mulmod(t, 1ull << 56, p);
     }
     uint64_t *blk = tables->data() + (size_t)c * kTableSlots * N;
-    uint64_t *phi = blk + kPhi * N, *phi_s = blk + kPhiShoup * N;
-    uint64_t *iphi = blk + kInvPhi * N, *iphi_s = blk + kInvPhiShoup * N;
+    uint64_t *phi = blk + kPhi * N, *iphi = blk + kInvPhi * N;
     // phi is a primitive 2N-th root: the 2^14-th root squared 13 - log2 N times.
     uint64_t root = kRoots2p14[c];
     for (int i = 0; i < 13 - (int)ps->log_n; i++) root = mulmod(root, root, p);
     t = 1;
     for (uint32_t i = 0; i < N; i++) {
-      phi[i] = t;
-      phi_s[i] = shoup_of(t, p);
+      put(phi, i, t, p);
       t = mulmod(t, root, p);
     }
-    const uint64_t inv_root = mulmod(t, phi[N - 1], p);  // phi^N * phi^(N-1) = phi^-1
-    t = mulmod(kInv8192[c], kMaxPolyDegree / N, p);       // N^-1
+    const uint64_t inv_root = mulmod(t, phi[2 * (N - 1)], p);  // phi^N * phi^(N-1) = phi^-1
+    t = mulmod(kInv8192[c], kMaxPolyDegree / N, p);              // N^-1
     for (uint32_t i = 0; i < N; i++) {
-      iphi[i] = t;
-      iphi_s[i] = shoup_of(t, p);
+      put(iphi, i, t, p);
       t = mulmod(t, inv_root, p);
     }
-    layer_powers(blk + kOmega * N, blk + kOmegaShoup * N, mulmod(root, root, p), N, p);
-    layer_powers(blk + kInvOmega * N, blk + kInvOmegaShoup * N, mulmod(inv_root, inv_root, p), N, p);
+    layer_powers(blk + kOmega * N, mulmod(root, root, p), N, p);
+    layer_powers(blk + kInvOmega * N, mulmod(inv_root, inv_root, p), N, p);
   }
   return true;
 }

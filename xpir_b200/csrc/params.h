@@ -16,17 +16,16 @@ extern const uint64_t kModuli[kMaxModuli];
 extern const uint64_t kRoots2p14[kMaxModuli];
 extern const uint64_t kInv8192[kMaxModuli];
 
-// Per-modulus table block, N words each, in this order (word offsets are multiples of N):
+// Per-modulus table block of four tables, N pairs of words each: a factor and its Shoup
+// factor floor(f 2^64 / p) side by side, so that one 16-byte load brings both.  The values
+// are the offsets in N words.
 enum TableSlot : uint32_t {
-  kPhi = 0,        // phi^i                       (crypto/NFLlib.cpp:94-101)
-  kPhiShoup,       // floor(phi^i 2^64 / p)
-  kOmega,          // forward twiddles, layer by layer: N/2 powers of w, N/4 of w^2, ...
-  kOmegaShoup,     //                               (crypto/NFLlib.hpp:571-586)
-  kInvPhi,         // N^-1 phi^-i                 (crypto/NFLlib.cpp:109-121)
-  kInvPhiShoup,
-  kInvOmega,       // inverse twiddles, same layout as kOmega
-  kInvOmegaShoup,
-  kTableSlots
+  kPhi = 0,       // phi^i                       (crypto/NFLlib.cpp:94-101)
+  kOmega = 2,     // forward twiddles, layer by layer: N/2 powers of w, N/4 of w^2, ...
+                  //                               (crypto/NFLlib.hpp:571-586)
+  kInvPhi = 4,    // N^-1 phi^-i                 (crypto/NFLlib.cpp:109-121)
+  kInvOmega = 6,  // inverse twiddles, same layout as kOmega
+  kTableSlots = 8
 };
 
 // Constants the kernels need per modulus, passed by value as a kernel argument.

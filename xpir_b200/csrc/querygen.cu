@@ -89,62 +89,75 @@ __device__ __forceinline__ void salsa20_block(const uint32_t key[8], uint64_t no
   for (int i = 0; i < 16; i++) out[i] = x[i] + in[i];
 }
 
+// The masked words of one Salsa20 block, 8 per block, as 64-bit words.
+__device__ __forceinline__ uint64_t word_of(const uint32_t (&w)[16], int k) {
+  return (uint64_t)w[2 * k] | (uint64_t)w[2 * k + 1] << 32;
+}
+
+template <int LOGN>
 __global__ void __launch_bounds__(256, 4) encrypt_kernel(const QueryGenArgs g, const uint64_t *__restrict__ sk,
-                                                      const uint64_t *__restrict__ sks,
-                                                      const uint64_t *__restrict__ tables, uint32_t N, uint32_t log_n,
-                                                      uint32_t m, const DevModuli dm, uint64_t *__restrict__ out) {
-  extern __shared__ uint64_t poly[];                     // N words, swizzled (the NTT's buffer)
-  uint32_t *noise = reinterpret_cast<uint32_t *>(poly + N);  // N words, [k][blk] (conflict-free)
-  const uint32_t nb = N / 8;                             // Salsa20 blocks of 8 words per poly
+                                                         const uint64_t *__restrict__ sks,
+                                                         const uint64_t *__restrict__ tables, uint32_t m,
+                                                         const DevModuli dm, uint64_t *__restrict__ out) {
+  constexpr uint32_t N = 1u << LOGN, nb = N / 8;             // Salsa20 blocks of 8 words per poly
+  extern __shared__ __align__(16) uint64_t poly[];           // N words, swizzled (the NTT's buffer)
+  uint32_t *noise = reinterpret_cast<uint32_t *>(poly + N);  // N words
   const uint64_t t = blockIdx.x;
   uint64_t ui = 0;
   for (uint32_t l = 0; l < g.d; l++) ui |= (g.one_slot[l] == t) ? 1 : 0;
   const uint64_t nonce_e = g.first_nonce + 2 * t, nonce_a = nonce_e + 1;
   // noise e (the same words for every modulus): word & mask, minus the bound when above it
   for (uint32_t blk = threadIdx.x; blk < nb; blk += blockDim.x) {
-    uint32_t w[16];
+    uint32_t w[16], e[8];
     salsa20_block(g.key, nonce_e, blk, w);
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-      uint64_t r = ((uint64_t)w[2 * k] | (uint64_t)w[2 * k + 1] << 32) & g.noise_mask;
+      uint64_t r = word_of(w, k) & g.noise_mask;
       if (r >= g.noise_bound) r -= g.noise_bound;
-      noise[k * nb + blk] = (uint32_t)r;  // read back by this thread only
+      e[k] = (uint32_t)r;
     }
+    reinterpret_cast<uint4 *>(noise)[2 * blk] = make_uint4(e[0], e[1], e[2], e[3]);
+    reinterpret_cast<uint4 *>(noise)[2 * blk + 1] = make_uint4(e[4], e[5], e[6], e[7]);
   }
+  __syncthreads();
   for (uint32_t c = 0; c < m; c++) {
     const uint64_t p = dm.p[c], p2 = p << 1;
     const uint64_t *tab = tables + (uint64_t)c * kTableSlots * N;
-    const uint64_t *phi = tab + kPhi * N, *phis = tab + kPhiShoup * N;
+    const ulonglong2 *phi = reinterpret_cast<const ulonglong2 *>(tab + kPhi * N);
     // amplified, plus the plaintext, twisted
-    for (uint32_t blk = threadIdx.x; blk < nb; blk += blockDim.x) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t i = blk * 8 + k;
-        uint64_t z = shoup_mul(noise[k * nb + blk], g.amp[c], g.amp_shoup[c], p) + (i == 0 ? ui : 0);
-        z -= (z >= p) ? p : 0;
-        if (z > p) z -= p;
-        poly[swz(i)] = shoup_mul(z, phi[i], phis[i], p);
-      }
-    }
-    __syncthreads();
-    ntt_lazy_rb<3>(poly, tab + kOmega * N, tab + kOmegaShoup * N, N, log_n, p,
-                   [&](uint32_t k) { return poly[swz(k)]; });
+    auto coefficient = [&](uint32_t i) -> uint64_t {
+      const ulonglong2 f = __ldg(phi + i);
+      uint64_t z = shoup_mul(noise[i], g.amp[c], g.amp_shoup[c], p) + (i == 0 ? ui : 0);
+      z -= (z >= p) ? p : 0;
+      if (z > p) z -= p;
+      return shoup_mul(z, f.x, f.y, p);
+    };
+    ntt_lazy<LOGN, false>(poly, reinterpret_cast<const ulonglong2 *>(tab + kOmega * N), p, coefficient);
     // uniform a: words [c*N, (c+1)*N) of the second call's stream
-    uint64_t *a_out = out + (t * 2 * m + c) * N, *b_out = out + (t * 2 * m + m + c) * N;
-    const uint64_t *s = sk + (uint64_t)c * N, *ss = sks + (uint64_t)c * N;
+    ulonglong2 *a_out = reinterpret_cast<ulonglong2 *>(out + (t * 2 * m + c) * N);
+    ulonglong2 *b_out = reinterpret_cast<ulonglong2 *>(out + (t * 2 * m + m + c) * N);
+    const ulonglong2 *s = reinterpret_cast<const ulonglong2 *>(sk + (uint64_t)c * N);
+    const ulonglong2 *ss = reinterpret_cast<const ulonglong2 *>(sks + (uint64_t)c * N);
     for (uint32_t blk = threadIdx.x; blk < nb; blk += blockDim.x) {
       uint32_t w[16];
       salsa20_block(g.key, nonce_a, (uint64_t)c * nb + blk, w);
+      const uint32_t at = swz(blk * 8);
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t i = blk * 8 + k;
-        uint64_t a = ((uint64_t)w[2 * k] | (uint64_t)w[2 * k + 1] << 32) & g.uniform_mask[c];
-        if (a >= p) a -= p;
-        uint64_t b = shoup_mac(poly[swz(i)], a, s[i], ss[i], p);
-        b -= (b >= p2) ? p2 : 0;
-        b -= (b >= p) ? p : 0;
-        a_out[i] = a;
-        b_out[i] = b;
+      for (int k = 0; k < 8; k += 2) {
+        const ulonglong2 key = __ldg(s + blk * 4 + k / 2), key_s = __ldg(ss + blk * 4 + k / 2);
+        ulonglong2 a, b;
+        a.x = word_of(w, k) & g.uniform_mask[c];
+        a.y = word_of(w, k + 1) & g.uniform_mask[c];
+        if (a.x >= p) a.x -= p;
+        if (a.y >= p) a.y -= p;
+        b.x = shoup_mac(poly[at ^ k], a.x, key.x, key_s.x, p);
+        b.y = shoup_mac(poly[at ^ (k + 1)], a.y, key.y, key_s.y, p);
+        b.x -= (b.x >= p2) ? p2 : 0;
+        b.x -= (b.x >= p) ? p : 0;
+        b.y -= (b.y >= p2) ? p2 : 0;
+        b.y -= (b.y >= p) ? p : 0;
+        a_out[blk * 4 + k / 2] = a;
+        b_out[blk * 4 + k / 2] = b;
       }
     }
     __syncthreads();  // the next modulus rewrites poly
@@ -258,10 +271,16 @@ extern "C" int xpir_b200_generate_query(xpir_b200_ctx *ctx, const uint8_t *prng_
     target = d_out;
   }
   const int smem = (int)(N * 8 + N * 4);  // the NTT's poly and the 32-bit noise words
-  if (e == cudaSuccess) e = allow_max_dynamic_smem((const void *)encrypt_kernel);
   if (e == cudaSuccess) {
-    encrypt_kernel<<<(unsigned)nq, 256, smem, st>>>(g, d_sk, d_sks, ctx->d_tables, N, ps.log_n, m, dm, target);
-    e = cudaGetLastError();
+#define XPIR_ENCRYPT(L)                                                                                     \
+  {                                                                                                         \
+    e = allow_max_dynamic_smem((const void *)encrypt_kernel<L>);                                            \
+    if (e == cudaSuccess) {                                                                                 \
+      encrypt_kernel<L><<<(unsigned)nq, 256, smem, st>>>(g, d_sk, d_sks, ctx->d_tables, m, dm, target);     \
+      e = cudaGetLastError();                                                                               \
+    }                                                                                                       \
+  }
+    XPIR_BY_DEGREE(ps.log_n, XPIR_ENCRYPT)
     ctx->launches++;
   }
   if (e == cudaSuccess && !out_on_device) e = cudaMemcpyAsync(query, d_out, nq * ct_bytes, cudaMemcpyDeviceToHost, st);
