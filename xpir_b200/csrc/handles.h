@@ -31,7 +31,7 @@ struct xpir_b200_ctx {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t query_copied = nullptr;
   xpir::ParamSet ps;           // b is set per database
-  uint64_t *d_tables = nullptr;  // also holds zero_poly and ws_part
+  uint64_t *d_tables = nullptr;  // also holds zero_poly and stop_flag
   std::mutex mu;
   std::atomic<uint64_t> launches{0};  // engine kernels launched (also counted off the lock)
   std::atomic<int> servers{0};         // servers with a lane on this context
@@ -73,10 +73,10 @@ struct xpir_b200_ctx {
 
 constexpr int kZeroHints = 1022;
 
-// Workspace of the residue sums' runs: 1.8 MiB per context, made with it, so that no reply
+// Workspace of the residue sums' runs: 3.8 MiB per context, taken with it, so that no reply
 // allocates it (a level takes as many runs as fit; the 100,000 x 4 KB level's 27 take 221,184
 // words).
-constexpr uint64_t kPartWords = 240000;
+constexpr uint64_t kPartWords = 500000;
 
 // Tile shape for a level shape: the autotuned one if any, else -1 (default).
 inline int tuned_tile(const xpir_b200_ctx *ctx, uint64_t P, uint64_t n_i, uint64_t groups) {
