@@ -142,21 +142,24 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
         row[i] = (int)(g * sh.n_i);
         poly[i] = (int)(j - g * sh.P);
       }
-      uint32_t t = 0;
+      uint32_t t = 0, st = 0, phase = 1;
       for (; t < tiles; ++t) {
-        const int s = (int)(t % NS);
         if (*quit) break;
         if (t % 64 == (uint32_t)NS && *(volatile int *)sh.stop) {
           *quit = 1;
           break;
         }
-        if (t >= (uint32_t)NS && !wait_or_quit(empty + s, (t / NS - 1) & 1, quit)) break;
-        mbar_arrive_expect_tx(full + s, (uint32_t)((S::kX + S::kQ) * 8));
+        if (t >= (uint32_t)NS && !wait_or_quit(empty + st, phase, quit)) break;
+        mbar_arrive_expect_tx(full + st, (uint32_t)((S::kX + S::kQ) * 8));
         const int slot = (int)(s0 + t * E);
 #pragma unroll
         for (int i = 0; i < C; i++)
-          tma_load_4d(xs + s * S::kX + i * E * W, &task.tm_db, (int)k0, (int)c, poly[i], row[i] + slot, full + s);
-        tma_load_4d(qs + s * S::kQ, &task.tm_q, (int)k0, (int)c, 0, slot, full + s);
+          tma_load_4d(xs + st * S::kX + i * E * W, &task.tm_db, (int)k0, (int)c, poly[i], row[i] + slot, full + st);
+        tma_load_4d(qs + st * S::kQ, &task.tm_q, (int)k0, (int)c, 0, slot, full + st);
+        if (++st == NS) {
+          st = 0;
+          phase ^= 1;
+        }
       }
       // Every issued copy must have landed before the CTA exits.
       const uint32_t first = t > (uint32_t)NS ? t - NS : 0;
@@ -175,18 +178,25 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
     for (int i = 0; i < C; i++) sum_clear(acc[h][i], ONE ? 0 : kBoundStart);
   bool bad = false, late = false;
   const uint32_t sum_tiles = (sum_end - s0) / E;
-  uint32_t t = 0;
-  for (; t < sum_tiles; ++t) {
-    if (__any_sync(~0u, bad)) {  // the whole warp stops
-      bad = true;
-      break;
+  uint32_t t = 0, st = 0, phase = 0;
+  // Waits for tile t; false (in the whole warp) when it must stop.
+  auto tile_ready = [&]() -> bool {
+    const bool ok = mbar_try_wait(full + st, phase) || wait_or_quit(full + st, phase, quit);
+    if (!__any_sync(~0u, bad || !ok)) return true;
+    late = !__all_sync(~0u, ok);
+    bad = __any_sync(~0u, bad);
+    return false;
+  };
+  auto tile_done = [&] {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + st);
+    if (++st == NS) {
+      st = 0;
+      phase ^= 1;
     }
-    const int s = (int)(t % NS);
-    if (!__all_sync(~0u, wait_or_quit(full + s, (t / NS) & 1, quit))) {
-      late = true;
-      break;
-    }
-    const uint64_t *xst = xs + s * S::kX + k, *qst = qs + s * S::kQ + k;
+  };
+  for (; t < sum_tiles && tile_ready(); ++t) {
+    const uint64_t *xst = xs + st * S::kX + k, *qst = qs + st * S::kQ + k;
     int32_t peak = 0;
 #pragma unroll
     for (int e = 0; e < E; e += 4) {
@@ -226,8 +236,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
       }
     }
     bad |= peak > kBoundMax;
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty + s);
+    tile_done();
   }
   const uint64_t mN = (uint64_t)sh.m * sh.N;
   const uint64_t at = (uint64_t)c * sh.N + k0 + k;
@@ -245,14 +254,8 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
       for (int i = 0; i < C; i++)
         tail[h][i] = sum_tiles ? ExactTail{sum_residue(acc[h][i], p, np, delta), sum_above(acc[h][i].bound), 0}
                                : ExactTail{0, 0, 0};
-    for (; t < tiles && !late; ++t) {
-      if (__any_sync(~0u, bad)) break;
-      const int s = (int)(t % NS);
-      if (!__all_sync(~0u, wait_or_quit(full + s, (t / NS) & 1, quit))) {
-        late = true;
-        break;
-      }
-      const uint64_t *xst = xs + s * S::kX + k, *qst = qs + s * S::kQ + k;
+    for (; t < tiles && !late && tile_ready(); ++t) {
+      const uint64_t *xst = xs + st * S::kX + k, *qst = qs + st * S::kQ + k;
       const uint32_t left = min((uint32_t)E, end - (s0 + t * E));
       for (uint32_t e = 0; e < left; e++) {
 #pragma unroll
@@ -264,8 +267,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
           for (int i = 0; i < C; i++) tail_step(tail[h][i], shoup_lazy_np(xst[(i * E + e) * W], y, ys, np), p);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(empty + s);
+      tile_done();
     }
     if (!bad && !late) {
       const bool zero_p = sh.idle && sh.zero_poly[at] != 0;
