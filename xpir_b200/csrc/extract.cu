@@ -37,6 +37,10 @@ namespace {
 
 constexpr uint32_t kMaxLiftModuli = 4;  // b < 128 bits per coefficient
 constexpr int kLimbs = kMaxLiftModuli + 1;
+// Ciphertexts from which one CTA per ciphertext fills the GPU, and the shared memory it may
+// take (two CTAs per SM; larger parameter sets keep the two kernels).
+constexpr uint64_t kFusedCiphertexts = 296;
+constexpr size_t kFusedSmem = 112 * 1024;
 
 // Mixed-radix constants: x = v0 + v1*M1 + ... with M_c = p_0*...*p_{c-1}.
 struct LiftConsts {
@@ -49,17 +53,34 @@ struct LiftConsts {
 // Exact reductions modulo one of XPIR's moduli (mod_word, mod_two_words) give the unique
 // residue the reference's GMP lift computes.
 //
-// x (its low nl of kLimbs little-endian limbs) mod p, from the top limb down; the loop is
-// unrolled over all limbs so that x stays in registers.
-__device__ __forceinline__ uint64_t limbs_mod_fast(const uint64_t (&x)[kLimbs], int nl, uint64_t p, uint64_t np,
-                                                   uint32_t delta) {
-  uint64_t r = 0;
+// x (its low NL little-endian limbs) mod p, from the top limb down.
+template <int NL>
+__device__ __forceinline__ uint64_t limbs_mod_fast(const uint64_t *x, uint64_t p, uint64_t np, uint32_t delta) {
+  uint64_t r = mod_word(x[NL - 1], p, np);
 #pragma unroll
-  for (int l = kLimbs - 1; l >= 0; l--) {
-    if (l == nl - 1) r = mod_word(x[l], p, np);
-    else if (l < nl - 1) r = mod_two_words(r, x[l], p, np, delta);
-  }
+  for (int l = NL - 2; l >= 0; l--) r = mod_two_words(r, x[l], p, np, delta);
   return r;
+}
+
+// b - a*s of one ciphertext and modulus, transformed back: coefficient k (before the N^-1
+// phi^-k scaling) is left in poly[swz(brev(k))].
+template <int LOGN>
+__device__ __forceinline__ void decrypt_poly(uint64_t *poly, const uint64_t *__restrict__ a,
+                                             const uint64_t *__restrict__ b, const uint64_t *__restrict__ s,
+                                             const uint64_t *__restrict__ ss, const uint64_t *__restrict__ tab,
+                                             uint64_t p) {
+  constexpr uint32_t N = 1u << LOGN, shift = 32 - LOGN;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {  // unrolled: several rows of loads in flight
+    const uint64_t temp = shoup_mac(0, a[i], s[i], ss[i], p);  // in [0, p)
+    const uint64_t y = (temp < p) ? p - temp : p - temp % p;
+    uint64_t z = b[i] + y;
+    z -= (z >= p) ? p : 0;
+    poly[swz(__brev(i) >> shift)] = z;
+  }
+  __syncthreads();
+  ntt_lazy<LOGN, false, true>(poly, reinterpret_cast<const ulonglong2 *>(tab + kInvOmega * N), p,
+                              [&](uint32_t k) { return poly[swz(k)]; });
 }
 
 template <int LOGN>
@@ -71,22 +92,10 @@ __global__ void __launch_bounds__(256, 4) decrypt_poly_kernel(const uint64_t *__
   constexpr uint32_t N = 1u << LOGN, shift = 32 - LOGN;
   extern __shared__ __align__(16) uint64_t poly[];
   const uint32_t c = blockIdx.y;
-  const uint64_t j = blockIdx.x;
-  const uint64_t p = dm.p[c];
-  const uint64_t *a = ct + (j * 2 * m + c) * N, *b = ct + (j * 2 * m + m + c) * N;
-  const uint64_t *s = sk + (uint64_t)c * N, *ss = sks + (uint64_t)c * N;
-#pragma unroll 4
-  for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {  // unrolled: several rows of loads in flight
-    const uint64_t temp = shoup_mac(0, a[i], s[i], ss[i], p);  // in [0, p)
-    const uint64_t y = (temp < p) ? p - temp : p - temp % p;
-    uint64_t z = b[i] + y;
-    z -= (z >= p) ? p : 0;
-    poly[swz(__brev(i) >> shift)] = z;
-  }
-  __syncthreads();
+  const uint64_t j = blockIdx.x, p = dm.p[c];
   const uint64_t *tab = tables + (uint64_t)c * kTableSlots * N;
-  ntt_lazy<LOGN, false, true>(poly, reinterpret_cast<const ulonglong2 *>(tab + kInvOmega * N), p,
-                              [&](uint32_t k) { return poly[swz(k)]; });
+  decrypt_poly<LOGN>(poly, ct + (j * 2 * m + c) * N, ct + (j * 2 * m + m + c) * N, sk + (uint64_t)c * N,
+                     sks + (uint64_t)c * N, tab, p);
   const ulonglong2 *iphi = reinterpret_cast<const ulonglong2 *>(tab + kInvPhi * N);
   uint64_t *o = res + (j * m + c) * N;
   // In output order (coalesced global loads and stores); the bit reversal is its own
@@ -97,42 +106,74 @@ __global__ void __launch_bounds__(256, 4) decrypt_poly_kernel(const uint64_t *__
   }
 }
 
+// One more modulus of the mixed radix: x += M_C * v with v in [0, p_C) such that x = residue
+// mod p_C.  Before it x < p_0*...*p_{C-1} < 2^(61C) has C limbs (as M_C), after it C + 1.
+template <int C, int M>
+__device__ __forceinline__ void lift_step(uint64_t (&x)[M], uint64_t residue, const LiftConsts &lc, const DevModuli &dm) {
+  const uint64_t p = dm.p[C], np = 0 - p;
+  const uint64_t r = mod_word(residue, p, np);
+  if constexpr (C == 0) {
+    x[0] = r;
+  } else {
+    uint64_t t = r + p - limbs_mod_fast<C>(x, p, np, (uint32_t)dm.shoup_delta[C]);
+    t = t >= p ? t - p : t;
+    const uint64_t v = shoup_mul(t, lc.inv[C], lc.inv_shoup[C], p);
+    unsigned __int128 carry = 0;
+#pragma unroll
+    for (int l = 0; l < C; l++) {
+      const unsigned __int128 s = (unsigned __int128)lc.M[C][l] * v + x[l] + carry;
+      x[l] = (uint64_t)s;
+      carry = s >> 64;
+    }
+    x[C] = (uint64_t)carry;
+  }
+}
+
+// The plaintext value of one coefficient from its M residues (residue(c), any 64-bit words):
+// mixed radix, centred, cut to `bits` bits.
+template <int M, class Residue>
+__device__ __forceinline__ unsigned __int128 lift(uint32_t bits, const LiftConsts &lc, const DevModuli &dm,
+                                                  Residue residue) {
+  uint64_t x[M];
+  lift_step<0>(x, residue(0), lc, dm);
+  if constexpr (M > 1) lift_step<1>(x, residue(1), lc, dm);
+  if constexpr (M > 2) lift_step<2>(x, residue(2), lc, dm);
+  if constexpr (M > 3) lift_step<3>(x, residue(3), lc, dm);
+  // centred: x - P when 2x > P
+  int cmp = 0;  // sign of 2x - P (x < P < 2^(61M): 2x fits the limbs)
+#pragma unroll
+  for (int l = M - 1; l >= 0; l--) {
+    const uint64_t x2 = (x[l] << 1) | (l ? x[l > 0 ? l - 1 : 0] >> 63 : 0);
+    if (cmp == 0 && x2 != lc.P[l]) cmp = x2 > lc.P[l] ? 1 : -1;
+  }
+  unsigned __int128 v = x[0], top = lc.P[0];
+  if constexpr (M > 1) {
+    v |= (unsigned __int128)x[1] << 64;
+    top |= (unsigned __int128)lc.P[1] << 64;
+  }
+  if (cmp > 0) v -= top;  // below 2^128: for one modulus the difference's high word is all ones
+  return v & ((((unsigned __int128)1) << bits) - 1);
+}
+
+// lift() for a modulus count known at run time (1..kMaxLiftModuli).
+template <class Residue>
+__device__ __forceinline__ unsigned __int128 lift_any(uint32_t m, uint32_t bits, const LiftConsts &lc,
+                                                      const DevModuli &dm, Residue residue) {
+  switch (m) {
+    case 1: return lift<1>(bits, lc, dm, residue);
+    case 2: return lift<2>(bits, lc, dm, residue);
+    case 3: return lift<3>(bits, lc, dm, residue);
+    default: return lift<4>(bits, lc, dm, residue);
+  }
+}
+
 __global__ void __launch_bounds__(256) lift_pack_kernel(const uint64_t *__restrict__ res, uint64_t nct, uint32_t N,
                                                         uint32_t m, uint32_t bits, const LiftConsts lc,
                                                         const DevModuli dm, unsigned long long *__restrict__ out) {
   const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (t >= nct * N) return;
   const uint64_t j = t / N, i = t % N;
-  uint64_t x[kLimbs] = {};
-#pragma unroll
-  for (uint32_t c = 0; c < kMaxLiftModuli; c++) {  // unrolled: static indexes into x and the constants
-    if (c >= m) break;
-    const uint64_t p = dm.p[c], np = 0 - p;
-    const uint32_t delta = (uint32_t)dm.shoup_delta[c];
-    const uint64_t r = mod_word(res[(j * m + c) * N + i], p, np);
-    // x < p_0*...*p_{c-1} < 2^(61c): ceil(61c/64) limbs
-    const uint64_t have = c ? limbs_mod_fast(x, (int)((61 * c + 63) / 64), p, np, delta) : 0;
-    uint64_t t = r + p - have;
-    t = t >= p ? t - p : t;
-    const uint64_t v = c ? shoup_mul(t, lc.inv[c], lc.inv_shoup[c], p) : r;
-    unsigned __int128 carry = 0;  // x += M_c * v
-#pragma unroll
-    for (int l = 0; l < kLimbs; l++) {
-      const unsigned __int128 s = (unsigned __int128)lc.M[c][l] * v + x[l] + carry;
-      x[l] = (uint64_t)s;
-      carry = s >> 64;
-    }
-  }
-  // centred: x - P when 2x > P
-  int cmp = 0;  // sign of 2x - P (x < P < 2^244: 2x fits the limbs)
-#pragma unroll
-  for (int l = kLimbs - 1; l >= 0; l--) {  // unrolled (static limb indexes: registers)
-    const uint64_t x2 = (x[l] << 1) | (l ? x[l - 1] >> 63 : 0);
-    if (cmp == 0 && x2 != lc.P[l]) cmp = x2 > lc.P[l] ? 1 : -1;
-  }
-  unsigned __int128 v = ((unsigned __int128)x[1] << 64) | x[0];
-  if (cmp > 0) v -= ((unsigned __int128)lc.P[1] << 64) | lc.P[0];
-  if (bits < 128) v &= (((unsigned __int128)1) << bits) - 1;
+  const unsigned __int128 v = lift_any(m, bits, lc, dm, [&](uint32_t c) { return res[(j * m + c) * N + i]; });
   // append at bit offset i*bits of ciphertext j's plaintext (bits*N/64 words per ciphertext)
   const uint64_t pos = (uint64_t)i * bits, words = (uint64_t)bits * N / 64;
   unsigned long long *w = out + j * words + (pos >> 6);
@@ -143,6 +184,64 @@ __global__ void __launch_bounds__(256) lift_pack_kernel(const uint64_t *__restri
   if (w0) atomicOr(w, (unsigned long long)w0);
   if (w1) atomicOr(w + 1, (unsigned long long)w1);
   if (w2) atomicOr(w + 2, (unsigned long long)w2);
+}
+
+// Decryption, lift and packing of one ciphertext per CTA: the moduli one after another, their
+// residues kept in shared memory (the last one's in registers), then each thread packs whole
+// words of the plaintext.  For many ciphertexts: the residues never reach HBM and no word is
+// written twice (decrypt_poly_kernel and lift_pack_kernel move 2 * m * N words more per
+// ciphertext, zero the output first and update it atomically).  Rows of `keep`: m - 1, and as
+// many as a value has words.  The output is `limit` bytes long.
+template <int LOGN>
+__global__ void __launch_bounds__(256, 4) extract_kernel(const uint64_t *__restrict__ ct,
+                                                         const uint64_t *__restrict__ sk,
+                                                         const uint64_t *__restrict__ sks,
+                                                         const uint64_t *__restrict__ tables, uint32_t m, uint32_t bits,
+                                                         const LiftConsts lc, const DevModuli dm,
+                                                         uint64_t *__restrict__ out, uint64_t limit) {
+  constexpr uint32_t N = 1u << LOGN, shift = 32 - LOGN;
+  extern __shared__ __align__(16) uint64_t poly[];
+  uint64_t *keep = poly + N;
+  const uint64_t j = blockIdx.x;
+  for (uint32_t c = 0; c < m; c++) {
+    const uint64_t p = dm.p[c];
+    decrypt_poly<LOGN>(poly, ct + (j * 2 * m + c) * N, ct + (j * 2 * m + m + c) * N, sk + (uint64_t)c * N,
+                       sks + (uint64_t)c * N, tables + (uint64_t)c * kTableSlots * N, p);
+    const ulonglong2 *iphi = reinterpret_cast<const ulonglong2 *>(tables + ((uint64_t)c * kTableSlots + kInvPhi) * N);
+    for (uint32_t k = threadIdx.x; k < N; k += blockDim.x) {
+      const ulonglong2 f = __ldg(iphi + k);
+      const uint64_t r = shoup_mul(poly[swz(__brev(k) >> shift)], f.x, f.y, p);
+      if (c + 1 < m) {
+        keep[c * N + k] = r;
+        continue;
+      }
+      const unsigned __int128 v = lift_any(m, bits, lc, dm, [&](uint32_t i) { return i + 1 < m ? keep[i * N + k] : r; });
+      keep[k] = (uint64_t)v;
+      if (bits > 64) keep[N + k] = (uint64_t)(v >> 64);
+    }
+    __syncthreads();
+  }
+  // Word w of the plaintext: bits 64w .. of the values, `bits` each.
+  const uint32_t words = bits * N / 64;
+  for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) {
+    const uint32_t from = w * 64;
+    uint32_t i = from / bits;
+    int at = (int)(i * bits) - (int)from;  // position of value i in the word
+    uint64_t v = 0;
+    for (; at < 64; i++, at += (int)bits) {
+      const uint64_t lo = keep[i], hi = bits > 64 ? keep[N + i] : 0;
+      if (at >= 0) v |= lo << at;
+      else if (at > -64) v |= lo >> -at | hi << (64 + at);
+      else v |= hi >> (-at - 64);
+    }
+    const uint64_t byte = (j * words + w) * 8;
+    if (byte + 8 <= limit) {
+      out[j * words + w] = v;
+    } else {
+      for (uint32_t k = 0; k < 8; k++)
+        if (byte + k < limit) reinterpret_cast<uint8_t *>(out)[byte + k] = (uint8_t)(v >> (8 * k));
+    }
+  }
 }
 
 // Limb helpers on the host.
@@ -260,6 +359,7 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
       e = cudaMemcpyAsync(d_in, replies, top * ct_words * 8, cudaMemcpyHostToDevice, st);
     level_in = d_in;
   }
+  bool delivered = false;  // the last level's kernel wrote the caller's buffer itself
   for (uint32_t lvl = d; lvl >= 1 && e == cudaSuccess; lvl--) {
     const uint64_t nbr = extract_count(aggregated_bytes, lvl, bits, N, m);
     uint64_t *res = nullptr, *out = nullptr;
@@ -267,11 +367,38 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
     // next level as its ciphertexts: size it for both.
     uint64_t out_words = nbr * abs_words + 3;
     if (lvl > 1) out_words = std::max<uint64_t>(out_words, extract_count(aggregated_bytes, lvl - 1, bits, N, m) * ct_words);
-    e = cudaMallocFromPoolAsync((void **)&res, nbr * mN * 8, ctx->pool, st);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&out, out_words * 8, ctx->pool, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, out_words * 8, st);
-    if (e == cudaSuccess && nbr > 0x7fffffffull) e = cudaErrorInvalidValue;
-    if (e == cudaSuccess) {
+    if (nbr > 0x7fffffffull) e = cudaErrorInvalidValue;
+    const uint32_t rows = std::max(m - 1, bits > 64 ? 2u : 1u);
+    const size_t fused_smem = (size_t)(1 + rows) * N * 8;
+    if (nbr >= kFusedCiphertexts && fused_smem <= kFusedSmem) {
+      // Only the words past the plaintext need zeroing, and the last level's plaintext can go
+      // straight to an aligned device buffer.
+      delivered = lvl == 1 && out_on_device && ((uintptr_t)plaintext & 7) == 0;
+      uint64_t *dst = (uint64_t *)plaintext, limit = aggregated_bytes;
+      if (!delivered) {
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&out, out_words * 8, ctx->pool, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(out + nbr * abs_words, 0, (out_words - nbr * abs_words) * 8, st);
+        dst = out;
+        limit = out_words * 8;
+      }
+      if (e == cudaSuccess) {
+#define XPIR_EXTRACT(L)                                                                                            \
+  {                                                                                                                \
+    e = allow_max_dynamic_smem((const void *)extract_kernel<L>);                                                   \
+    if (e == cudaSuccess) {                                                                                        \
+      extract_kernel<L><<<(unsigned)nbr, 256, fused_smem, st>>>(level_in, d_sk, d_sks, ctx->d_tables, m, bits, lc, \
+                                                              dm, dst, limit);                                     \
+      e = cudaGetLastError();                                                                                      \
+    }                                                                                                              \
+  }
+        XPIR_BY_DEGREE(ps.log_n, XPIR_EXTRACT)
+        ctx->launches++;
+      }
+    } else {
+      if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&res, nbr * mN * 8, ctx->pool, st);
+      if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&out, out_words * 8, ctx->pool, st);
+      if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, out_words * 8, st);
+      if (e == cudaSuccess) {
 #define XPIR_DECRYPT(L)                                                                                           \
   {                                                                                                               \
     e = allow_max_dynamic_smem((const void *)decrypt_poly_kernel<L>);                                             \
@@ -281,22 +408,23 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
       e = cudaGetLastError();                                                                                     \
     }                                                                                                             \
   }
-      XPIR_BY_DEGREE(ps.log_n, XPIR_DECRYPT)
+        XPIR_BY_DEGREE(ps.log_n, XPIR_DECRYPT)
+      }
+      if (e == cudaSuccess) {
+        const uint64_t threads = nbr * N;
+        lift_pack_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(res, nbr, N, m, bits, lc, dm,
+                                                                             (unsigned long long *)out);
+        e = cudaGetLastError();
+        ctx->launches += 2;
+      }
+      cudaFreeAsync(res, st);
     }
-    if (e == cudaSuccess) {
-      const uint64_t threads = nbr * N;
-      lift_pack_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(res, nbr, N, m, bits, lc, dm,
-                                                                           (unsigned long long *)out);
-      e = cudaGetLastError();
-      ctx->launches += 2;
-    }
-    cudaFreeAsync(res, st);
     // This level's plaintext is the next level's ciphertexts.
     if (d_out) cudaFreeAsync(d_out, st);
     d_out = out;
     level_in = out;
   }
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && !delivered)
     e = cudaMemcpyAsync(plaintext, d_out, aggregated_bytes,
                         out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st);
   cleanup();
