@@ -283,14 +283,14 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
         cudaFree(ctx->ws_a);
         ctx->ws_a = nullptr;
         ctx->ws_a_bytes = 0;
-        if ((e = cudaMalloc(&ctx->ws_a, z.ws_a)) != cudaSuccess) return finish(e);
+        if ((e = allocate(ctx, &ctx->ws_a, z.ws_a)) != cudaSuccess) return finish(e);
         ctx->ws_a_bytes = z.ws_a;
       }
       if (z.ws_b > ctx->ws_b_bytes) {
         cudaFree(ctx->ws_b);
         ctx->ws_b = nullptr;
         ctx->ws_b_bytes = 0;
-        if ((e = cudaMalloc(&ctx->ws_b, z.ws_b)) != cudaSuccess) return finish(e);
+        if ((e = allocate(ctx, &ctx->ws_b, z.ws_b)) != cudaSuccess) return finish(e);
         ctx->ws_b_bytes = z.ws_b;
       }
       wa = ctx->ws_a;
@@ -325,8 +325,8 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   auto plan = std::make_shared<BatchPlan>();
   plan->key = key;
   for (const Group &g : groups) plan->db_ids.push_back(g.db->id);
-  e = cudaMalloc(&plan->ws_a, std::max<size_t>(z.ws_a, 256));
-  if (e == cudaSuccess) e = cudaMalloc(&plan->ws_b, std::max<size_t>(z.ws_b, 256));
+  e = allocate(ctx, &plan->ws_a, std::max<size_t>(z.ws_a, 256));
+  if (e == cudaSuccess) e = allocate(ctx, &plan->ws_b, std::max<size_t>(z.ws_b, 256));
   // Two tables: the graph copies the first from host_tasks at every replay, so a repeat of the
   // batch slot by slot fills the second.
   if (e == cudaSuccess) e = cudaMalloc(&plan->dev_tasks, 2 * z.tasks * sizeof(ReplyTask));
@@ -378,8 +378,8 @@ extern "C" int xpir_b200_autotune(xpir_b200_ctx *ctx, const xpir_b200_db *db, ui
   }
   uint64_t *rep = nullptr, *next = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  e = cudaMalloc(&rep, rep_max);
-  if (e == cudaSuccess && next_max) e = cudaMalloc(&next, next_max);
+  e = allocate(ctx, (void **)&rep, rep_max);
+  if (e == cudaSuccess && next_max) e = allocate(ctx, (void **)&next, next_max);
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   *ctx->status_host = 0;

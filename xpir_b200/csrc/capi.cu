@@ -38,14 +38,14 @@ int cuda_status(cudaError_t e) {
     if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
-int grow(void **buf, size_t *have, size_t need) {
+int grow(xpir_b200_ctx *ctx, void **buf, size_t *have, size_t need) {
   if (need <= *have) return XPIR_B200_OK;
   if (*buf) {
     XPIR_TRY(cudaFree(*buf));
     *buf = nullptr;
     *have = 0;
   }
-  XPIR_TRY(cudaMalloc(buf, need));
+  XPIR_TRY(allocate(ctx, buf, need));
   *have = need;
   return XPIR_B200_OK;
 }
@@ -250,6 +250,7 @@ int xpir_b200_ctx_destroy(xpir_b200_ctx *ctx) {
     delete db;
   }
   ctx->dbs.clear();
+  drop_spare(ctx);
   cudaFree(ctx->d_tables);
   give_part(ctx->ws_part);
   cudaFree(ctx->ws_query);
@@ -356,7 +357,16 @@ int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, uint64_t nb_el
   db->b = b;
   db->alpha = alpha;
   db->element_bytes = element_bytes;
-  cudaError_t e = cudaMalloc(&db->d_polys, (words + 2) * sizeof(uint64_t));  // the last two: zero_seen
+  db->alloc_bytes = (words + 2) * sizeof(uint64_t);  // the last two: zero_seen
+  cudaError_t e = cudaSuccess;
+  if (ctx->spare && db->alloc_bytes <= ctx->spare_bytes && db->alloc_bytes >= ctx->spare_bytes / 2) {
+    db->d_polys = (uint64_t *)ctx->spare;
+    db->alloc_bytes = ctx->spare_bytes;
+    ctx->spare = nullptr;
+    ctx->spare_bytes = 0;
+  } else {
+    e = allocate(ctx, (void **)&db->d_polys, db->alloc_bytes);
+  }
   if (e != cudaSuccess) {
     delete db;
     return cuda_status(e);
@@ -364,7 +374,7 @@ int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, uint64_t nb_el
   const uint8_t *src = (const uint8_t *)elements;
   void *staging = nullptr;
   if (!src_on_device) {
-    e = cudaMalloc(&staging, src_bytes);
+    e = allocate(ctx, &staging, src_bytes);
     if (e == cudaSuccess) e = cudaMemcpyAsync(staging, elements, src_bytes, cudaMemcpyHostToDevice, ctx->stream);
     src = (const uint8_t *)staging;
   }
@@ -406,7 +416,13 @@ int xpir_b200_db_free(xpir_b200_db *db) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   drop_plans_of(ctx, db->id);
-  cudaFree(db->d_polys);
+  if (db->alloc_bytes <= kSpareBytes && db->alloc_bytes > ctx->spare_bytes) {
+    drop_spare(ctx);
+    ctx->spare = db->d_polys;
+    ctx->spare_bytes = db->alloc_bytes;
+  } else {
+    cudaFree(db->d_polys);
+  }
   if (db->hint) ctx->free_hints.push_back(db->hint);
   delete db;
   return XPIR_B200_OK;
@@ -472,8 +488,8 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
   if (capacity_bytes < final_bytes) return XPIR_B200_ERR_ARG;
   if (!out_on_device) need_a = final_bytes > need_a ? final_bytes : need_a;
   int rc;
-  if ((rc = grow(&ctx->ws_a, &ctx->ws_a_bytes, need_a)) != XPIR_B200_OK) return rc;
-  if ((rc = grow(&ctx->ws_b, &ctx->ws_b_bytes, need_b)) != XPIR_B200_OK) return rc;
+  if ((rc = grow(ctx, &ctx->ws_a, &ctx->ws_a_bytes, need_a)) != XPIR_B200_OK) return rc;
+  if ((rc = grow(ctx, &ctx->ws_b, &ctx->ws_b_bytes, need_b)) != XPIR_B200_OK) return rc;
 
   const uint64_t *dq = (const uint64_t *)query;
   const bool split_copy = !query_on_device && d > 1;
@@ -487,7 +503,7 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
     }
   } copy_guard{ctx->copy_stream, split_copy};
   if (!query_on_device) {
-    if ((rc = grow(&ctx->ws_query, &ctx->ws_query_bytes, total_ct * ct_bytes)) != XPIR_B200_OK) return rc;
+    if ((rc = grow(ctx, &ctx->ws_query, &ctx->ws_query_bytes, total_ct * ct_bytes)) != XPIR_B200_OK) return rc;
     // The first level's ciphertexts on the context's stream; the other levels' on the copy
     // stream, so that the first level's reply runs while they cross PCIe (the level loop
     // waits for them before level 2).

@@ -345,8 +345,8 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
     cudaFreeAsync(d_res, st);
     cudaFreeAsync(d_out, st);
   };
-  e = cudaMallocFromPoolAsync((void **)&d_sk, mN * 8, ctx->pool, st);
-  if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&d_sks, mN * 8, ctx->pool, st);
+  e = pool_allocate(ctx, (void **)&d_sk, mN * 8);
+  if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&d_sks, mN * 8);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_sk, secret_key, mN * 8, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
     e = launch_key_shoup(d_sk, d_sks, N, m, dm, st);
@@ -354,7 +354,7 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
   }
   const uint64_t *level_in = (const uint64_t *)replies;
   if (e == cudaSuccess && !replies_on_device) {
-    e = cudaMallocFromPoolAsync((void **)&d_in, top * ct_words * 8, ctx->pool, st);
+    e = pool_allocate(ctx, (void **)&d_in, top * ct_words * 8);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(d_in, replies, top * ct_words * 8, cudaMemcpyHostToDevice, st);
     level_in = d_in;
@@ -376,7 +376,7 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
       delivered = lvl == 1 && out_on_device && ((uintptr_t)plaintext & 7) == 0;
       uint64_t *dst = (uint64_t *)plaintext, limit = aggregated_bytes;
       if (!delivered) {
-        if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&out, out_words * 8, ctx->pool, st);
+        if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&out, out_words * 8);
         if (e == cudaSuccess) e = cudaMemsetAsync(out + nbr * abs_words, 0, (out_words - nbr * abs_words) * 8, st);
         dst = out;
         limit = out_words * 8;
@@ -395,8 +395,8 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
         ctx->launches++;
       }
     } else {
-      if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&res, nbr * mN * 8, ctx->pool, st);
-      if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&out, out_words * 8, ctx->pool, st);
+      if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&res, nbr * mN * 8);
+      if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&out, out_words * 8);
       if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, out_words * 8, st);
       if (e == cudaSuccess) {
 #define XPIR_DECRYPT(L)                                                                                           \

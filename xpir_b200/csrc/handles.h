@@ -53,6 +53,11 @@ struct xpir_b200_ctx {
   // mapped pinned memory: [0] kernel status, [1] redo (SumLevelArgs), then kZeroHints ints
   // that databases hold one of each (xpir_b200_db::hint)
   int *status_host = nullptr;
+  // The polys of the last freed database (at most kSpareBytes), for the next import: mapping
+  // and unmapping 655 MB costs more than importing them.  Released with the context, and when
+  // an allocation of this context fails.
+  void *spare = nullptr;
+  size_t spare_bytes = 0;
   int *status_dev = nullptr;
   uint64_t *zero_poly = nullptr;  // [m][N]: import of a zero bit stream
   int *stop_flag = nullptr;       // SumLevelArgs::stop
@@ -72,6 +77,7 @@ struct xpir_b200_ctx {
 };
 
 constexpr int kZeroHints = 1022;
+constexpr size_t kSpareBytes = 1ull << 30;
 
 // Workspace of the residue sums' runs: 3.8 MiB per context, taken with it, so that no reply
 // allocates it (a level takes as many runs as fit; the 100,000 x 4 KB level's 27 take 221,184
@@ -88,6 +94,7 @@ struct xpir_b200_db {
   xpir_b200_ctx *ctx = nullptr;
   uint64_t id = 0;  // unique per import in this process (never reused, unlike the address)
   uint64_t *d_polys = nullptr;
+  size_t alloc_bytes = 0;  // of d_polys
   uint64_t n_agg = 0;
   uint64_t P = 0;
   uint32_t b = 0;
@@ -117,6 +124,35 @@ inline xpir::SumLevelArgs sum_args(const xpir_b200_ctx *ctx, uint64_t n_real, ui
 struct xpir_b200_request;
 
 namespace xpir {
+// Gives the context's spare block back to the device (the caller holds ctx->mu).
+inline void drop_spare(xpir_b200_ctx *ctx) {
+  cudaFree(ctx->spare);
+  ctx->spare = nullptr;
+  ctx->spare_bytes = 0;
+}
+
+// cudaMalloc that does so when memory is short.
+inline cudaError_t allocate(xpir_b200_ctx *ctx, void **buf, size_t bytes) {
+  cudaError_t e = cudaMalloc(buf, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->spare) {
+    (void)cudaGetLastError();
+    drop_spare(ctx);
+    e = cudaMalloc(buf, bytes);
+  }
+  return e;
+}
+
+// The same for the context's stream-ordered pool.
+inline cudaError_t pool_allocate(xpir_b200_ctx *ctx, void **buf, size_t bytes) {
+  cudaError_t e = cudaMallocFromPoolAsync(buf, bytes, ctx->pool, ctx->stream);
+  if (e == cudaErrorMemoryAllocation && ctx->spare) {
+    (void)cudaGetLastError();
+    drop_spare(ctx);
+    e = cudaMallocFromPoolAsync(buf, bytes, ctx->pool, ctx->stream);
+  }
+  return e;
+}
+
 // Records a CUDA error as the calling thread's xpir_b200_last_cuda_error().
 void note_cuda_error(cudaError_t e);
 }  // namespace xpir

@@ -258,8 +258,8 @@ extern "C" int xpir_b200_generate_query(xpir_b200_ctx *ctx, const uint8_t *prng_
   if (e != cudaSuccess) return status_of(e);
   cudaStream_t st = ctx->stream;
   uint64_t *d_sk = nullptr, *d_sks = nullptr, *d_out = nullptr;
-  e = cudaMallocFromPoolAsync((void **)&d_sk, mN * 8, ctx->pool, st);
-  if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&d_sks, mN * 8, ctx->pool, st);
+  e = pool_allocate(ctx, (void **)&d_sk, mN * 8);
+  if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&d_sks, mN * 8);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_sk, secret_key, mN * 8, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
     e = launch_key_shoup(d_sk, d_sks, N, m, dm, st);
@@ -267,7 +267,7 @@ extern "C" int xpir_b200_generate_query(xpir_b200_ctx *ctx, const uint8_t *prng_
   }
   uint64_t *target = (uint64_t *)query;
   if (e == cudaSuccess && !out_on_device) {
-    e = cudaMallocFromPoolAsync((void **)&d_out, nq * ct_bytes, ctx->pool, st);
+    e = pool_allocate(ctx, (void **)&d_out, nq * ct_bytes);
     target = d_out;
   }
   const int smem = (int)(N * 8 + N * 4);  // the NTT's poly and the 32-bit noise words
@@ -309,7 +309,7 @@ extern "C" int xpir_b200_generate_secret_key(xpir_b200_ctx *ctx, const uint8_t *
   if (e != cudaSuccess) return status_of(e);
   cudaStream_t st = ctx->stream;
   uint64_t *d_sk = nullptr;
-  e = cudaMallocFromPoolAsync((void **)&d_sk, mN * 8, ctx->pool, st);
+  e = pool_allocate(ctx, (void **)&d_sk, mN * 8);
   if (e == cudaSuccess) {
     keygen_kernel<<<dim3((ps.N / 8 + 255) / 256, ps.m), 256, 0, st>>>(g, nonce, ps.N, dm, d_sk);
     e = cudaGetLastError();
