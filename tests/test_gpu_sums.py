@@ -27,6 +27,10 @@ SHAPES = [
     (1024, 1, [6, 10, 9], 1, 150, 300),  # idle elements inside, after and between second-level groups
     (1024, 1, [6, 10, 9], 1, 180, 300),  # 30 live of 90: the second level's groups are whole
     (1024, 2, [5, 8, 3, 4], 1, 27, 300),  # four levels
+    (1024, 1, [700], 1, 700, 5200),      # three columns per CTA, several runs
+    (512, 2, [700, 1], 3, 2100, 2500),   # the same with two moduli and aggregation
+    (512, 2, [133, 300], 1, 39870, 60),  # four columns per CTA, a partial last group
+    (512, 2, [128, 301], 1, 38528, 60),  # four columns per CTA, three of the last block empty
 ]
 
 

@@ -21,9 +21,7 @@
 // warp scheduler and the additions around it hardly overlap with it: a word and half cost
 // four of those and about twelve other instructions (32 cycles), where the slot-by-slot
 // kernel spends 56 on a Shoup factor and a Shoup product alone.  1,048,576 x 256 B in 16s:
-// level 1 2.47 -> 1.65 ms.  Two columns per CTA share the query words' preparation; three and
-// four were slower (register spills or too few warps: 206..290 against 189 us on a level of
-// 32 groups), as were 28 tail slots against 12 (245 against 239).
+// level 1 2.47 -> 1.50 ms.  Up to four columns per CTA share the query words' preparation.
 //
 // What the sums cannot decide sets *redo, and the caller repeats the call slot by slot.  A
 // CTA that finds such a word stops at once, so a query of unreduced words costs one tile.
@@ -442,14 +440,29 @@ cudaError_t launch_sum(const ReplyTask &one, const ReplyTask *dev, const SumShap
     }                                                                                               \
   }
 
-// By column count.  Three CTAs of four warps per SM hide the TMA's latency; their rings (72 and
-// 64 KB) and registers fill an SM.
+constexpr uint32_t kMaxRuns = 64;
+constexpr uint64_t kLongSlots = 128;
+
+// By column count.  Three CTAs of four warps per SM hide the TMA's latency with one and two
+// columns; their rings (72 and 64 KB) and registers fill an SM.  Three and four columns take
+// 80 and 96 KB and 168 registers: two CTAs.
 const SumEntry kSums[] = {
     XPIR_SUM(128, 1, 8, 3, 3),
     XPIR_SUM(128, 2, 8, 2, 3),
+    XPIR_SUM(128, 3, 8, 2, 2),
+    XPIR_SUM(128, 4, 8, 2, 2),
 };
-constexpr int kMaxSumColumns = 2;
-constexpr uint32_t kMaxRuns = 64;
+
+// Columns per CTA.  Four share the query words' preparation best, but leave too few CTAs and a
+// longer tail on small or short levels (us with two / four: 1,024 slots of 64 groups, N=4096
+// 2085 / 1903; 61 slots of 110 columns 161 / 174; 1,000 slots of 7 polys, N=1024 39 / 43).
+const SumEntry &sum_entry(uint32_t mN, uint64_t cols, uint64_t n_eff, uint64_t ntasks) {
+  if (cols == 3 && n_eff >= kLongSlots) return kSums[2];
+  const uint64_t ctas4 = mN / 128 * ((cols + 3) / 4) * ntasks;
+  if (cols >= 4 && n_eff >= kLongSlots && ctas4 >= 592) return kSums[3];
+  return kSums[cols == 1 ? 0 : 1];
+}
+
 
 int sum_sm_count() {
   static int cache[64] = {};
@@ -495,8 +508,8 @@ bool sum_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_live, u
   if (live_groups == 0 || ps.N % 128 != 0 || n_eff >= (1u << 30) || live_groups * P >= (1u << 30) ||
       !reply_level_supported(ps, n_live, n_i, live_groups) || ntasks > 65535 || live_groups * P > 65535)
     return false;
-  const SumEntry &entry = kSums[std::min<uint64_t>(kMaxSumColumns, live_groups * P) - 1];
-  const uint64_t ctas = (uint64_t)ps.m * ps.N / entry.W * ((live_groups * P + entry.C - 1) / entry.C) * ntasks;
+  const uint64_t cols = live_groups * P;  // in CTAs of 128 coefficients and two columns
+  const uint64_t ctas = (uint64_t)ps.m * ps.N / 128 * ((cols + 1) / 2) * ntasks;
   if (n_live * 2 < n_real) return true;
   return n_eff >= 600 || (n_eff >= kTailSlots && ctas >= (P > 1 ? 250u : 500u)) || (n_eff >= 96 && ctas >= 250);
 }
@@ -551,7 +564,7 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
     const uint64_t last_real = groups == 1 ? std::min(a.n_i, real) : a.n_i;
     sh.idle = last_real - sh.n_eff;
     sh.pad = a.n_i - last_real;
-    const SumEntry &entry = kSums[std::min<uint64_t>(kMaxSumColumns, sh.cols) - 1];
+    const SumEntry &entry = sum_entry((uint32_t)mN, sh.cols, sh.n_eff, ntasks);
     sh.slices = (uint32_t)(mN / entry.W);
     sh.col_blocks = (uint32_t)((sh.cols + entry.C - 1) / entry.C);
     sh.prefix = sh.n_eff > kTailSlots ? (sh.n_eff - kTailSlots) / entry.E * entry.E : 0;
