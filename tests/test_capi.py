@@ -110,6 +110,16 @@ def test_residue_sums_equal_chain_host(tmp_path):
     assert out.stdout.startswith("ok")
 
 
+def test_short_shoup_products_host(tmp_path):
+    """The Shoup product for small x and for factor 1 equals the general one."""
+    exe = tmp_path / "test_shoup_small"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-o", str(exe), str(ROOT / "tests" / "cpp" / "test_shoup_small.cpp"),
+                    str(ROOT / "xpir_b200" / "csrc" / "params.cpp")], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.startswith("ok")
+
+
 def test_admission_and_continuous_batching_host(tmp_path):
     """The serving loop's queueing rules (xpir_b200/csrc/admission.h) under a fake executor:
     FIFO per lane, budget never exceeded, oversize refused, batches formed from arrivals,

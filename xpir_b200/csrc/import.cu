@@ -139,10 +139,12 @@ __global__ void __launch_bounds__(T, MINB) import_kernel(const AggSource src, co
     const ulonglong2 f = __ldg(phi + k);
     const uint32_t pos = rel0 + k * b;
     uint64_t x = staged_bits(st, pos, mask_lo, mask_hi);
+    if (nsub == 1 && b <= 32) return shoup_mul_small((uint32_t)x, f.x, f.y, p);
     for (uint32_t t = 1; t < nsub; t++) {
       const int bits = t + 1 < nsub ? 56 : last_bits;
-      x += shoup_mul(staged_bits(st, pos + 56 * t, low_mask(bits), low_mask(bits - 32)), dm.crt[c][t],
-                     dm.crt_shoup[c][t], p);
+      const uint64_t sub = staged_bits(st, pos + 56 * t, low_mask(bits), low_mask(bits - 32));
+      x += bits <= 32 ? shoup_mul_small((uint32_t)sub, dm.crt[c][t], dm.crt_shoup[c][t], p)
+                      : shoup_mul(sub, dm.crt[c][t], dm.crt_shoup[c][t], p);
     }
     return shoup_mul(x, f.x, f.y, p);
   };

@@ -103,6 +103,22 @@ XPIR_HD uint64_t shoup_lazy(uint64_t x, uint64_t y, uint64_t ys, uint64_t p) {
 #endif
 }
 
+// The same product for x below 2^32: the quotient fits 32 bits too, and four of the ten
+// 32-bit products fall away.
+XPIR_HD uint64_t shoup_lazy_small_np(uint32_t x, uint64_t y, uint64_t ys, uint64_t np) {
+#if defined(__CUDA_ARCH__)
+  const uint32_t lo = __umulhi(x, (uint32_t)ys);
+#else
+  const uint32_t lo = (uint32_t)(((uint64_t)x * (uint32_t)ys) >> 32);
+#endif
+  const uint32_t q = (uint32_t)(((uint64_t)x * (uint32_t)(ys >> 32) + lo) >> 32);
+  const uint64_t r = (uint64_t)x * (uint32_t)y + (uint64_t)q * (uint32_t)np;
+  return r + ((uint64_t)(x * (uint32_t)(y >> 32) + q * (uint32_t)(np >> 32)) << 32);
+}
+
+// And for y = 1 (ys = 8 for every XPIR modulus), any x: the quotient is x >> 61.
+XPIR_HD uint64_t shoup_lazy_one_np(uint64_t x, uint64_t np) { return x + (x >> 61) * np; }
+
 // A value the compiler cannot see through (a register move on the device).
 XPIR_HD uint64_t opaque(uint64_t v) {
 #if defined(__CUDA_ARCH__)
@@ -115,6 +131,12 @@ XPIR_HD uint64_t opaque(uint64_t v) {
 // subtraction.
 XPIR_HD uint64_t shoup_mul(uint64_t x, uint64_t y, uint64_t ys, uint64_t p) {
   uint64_t r = shoup_lazy(x, y, ys, p);
+  return r >= p ? r - p : r;
+}
+
+// mulmodShoup for x below 2^32.
+XPIR_HD uint64_t shoup_mul_small(uint32_t x, uint64_t y, uint64_t ys, uint64_t p) {
+  const uint64_t r = shoup_lazy_small_np(x, y, ys, 0 - p);
   return r >= p ? r - p : r;
 }
 

@@ -48,13 +48,15 @@ __device__ __forceinline__ void ntt_layer(uint64_t (&x)[8], uint32_t base, const
   const ulonglong2 *t = tw + off + (base & (half - 1));
 #pragma unroll
   for (uint32_t k = 0; k < (1u << RB); k++) {
-    const ulonglong2 w = __ldg(t + (k << LO));
+    const bool one = LO == 0 && k == 0;  // every thread's twiddle is the layer's first power, 1
+    const ulonglong2 w = one ? make_ulonglong2(1, 8) : __ldg(t + (k << LO));
 #pragma unroll
     for (uint32_t r = k; r < 8; r += 1u << RB) {
       if (r & (1u << RB)) continue;
       const uint64_t u0 = x[r], u1 = x[r | (1u << RB)];
       x[r] = less_2p<ANY>(u0 + u1, p2);
-      x[r | (1u << RB)] = shoup_lazy_np(u0 - u1 + p2, w.x, w.y, np);
+      const uint64_t t1 = u0 - u1 + p2;
+      x[r | (1u << RB)] = one ? shoup_lazy_one_np(t1, np) : shoup_lazy_np(t1, w.x, w.y, np);
     }
   }
 }

@@ -95,7 +95,7 @@ __device__ __forceinline__ uint64_t word_of(const uint32_t (&w)[16], int k) {
 }
 
 template <int LOGN>
-__global__ void __launch_bounds__(256, 4) encrypt_kernel(const QueryGenArgs g, const uint64_t *__restrict__ sk,
+__global__ void __launch_bounds__(256, 3) encrypt_kernel(const QueryGenArgs g, const uint64_t *__restrict__ sk,
                                                          const uint64_t *__restrict__ sks,
                                                          const uint64_t *__restrict__ tables, uint32_t m,
                                                          const DevModuli dm, uint64_t *__restrict__ out) {
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256, 4) encrypt_kernel(const QueryGenArgs g, c
     // amplified, plus the plaintext, twisted
     auto coefficient = [&](uint32_t i) -> uint64_t {
       const ulonglong2 f = __ldg(phi + i);
-      uint64_t z = shoup_mul(noise[i], g.amp[c], g.amp_shoup[c], p) + (i == 0 ? ui : 0);
+      uint64_t z = shoup_mul_small(noise[i], g.amp[c], g.amp_shoup[c], p) + (i == 0 ? ui : 0);
       z -= (z >= p) ? p : 0;
       if (z > p) z -= p;
       return shoup_mul(z, f.x, f.y, p);
