@@ -194,8 +194,6 @@ template <int LOGN, int T, bool ALIAS, int MINB>
 cudaError_t launch_import_n(const AggSource &src, const ImportShape &sh, const DevModuli &dm, const uint64_t *tables,
                             uint64_t *out, cudaStream_t stream) {
   auto kern = import_kernel<LOGN, T, ALIAS, MINB>;
-  const cudaError_t e = allow_max_dynamic_smem((const void *)kern);
-  if (e != cudaSuccess) return e;
   const size_t words = ALIAS ? std::max(sh.stage_words, sh.N) : sh.stage_words + sh.N;
   kern<<<dim3((unsigned)sh.polys, sh.m), T, words * 8, stream>>>(src, sh, dm, tables, out);
   return cudaGetLastError();
@@ -224,8 +222,6 @@ template <int LOGN>
 cudaError_t launch_zero_fill(const ImportShape &sh, const DevModuli &dm, const uint64_t *tables, uint64_t *out,
                              uint64_t count, unsigned blocks, cudaStream_t stream) {
   auto kern = import_zero_fill_kernel<LOGN>;
-  const cudaError_t e = allow_max_dynamic_smem((const void *)kern);
-  if (e != cudaSuccess) return e;
   kern<<<dim3(blocks, sh.m), ntt_threads(sh.N), (size_t)sh.N * 8, stream>>>(sh, dm, tables, out, count);
   return cudaGetLastError();
 }
@@ -289,12 +285,12 @@ cudaError_t launch_zero_poly(const ParamSet &ps, const DevModuli &dm, const uint
 }
 
 // Loads the import kernels on the current device (lazy module loading would otherwise do
-// it, and reserve their device memory, at their first launch).
+// it, and reserve their device memory, at their first launch) and lets them take any amount
+// of shared memory.
 cudaError_t preload_import_kernels() {
-  cudaFuncAttributes fa;
   for (const ImportEntry &entry : kImports)
     for (const void *k : entry.kernels) {
-      const cudaError_t e = cudaFuncGetAttributes(&fa, k);
+      const cudaError_t e = allow_max_dynamic_smem(k);
       if (e != cudaSuccess) return e;
     }
   return cudaSuccess;

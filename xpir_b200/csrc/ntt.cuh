@@ -23,9 +23,13 @@ namespace xpir {
 
 // Position of coefficient idx in a swizzled shared-memory polynomial: the low 4 bits of
 // the word index XORed with bits 7..4, so that the passes of ntt_lazy (and the callers'
-// coefficient-order loops) read and write shared memory with few or no bank conflicts.
-// Linear over XOR, so swz(a | b) = swz(a) ^ swz(b) for disjoint bits.
-__host__ __device__ constexpr uint32_t swz(uint32_t idx) { return idx ^ ((idx >> 4) & 15u); }
+// coefficient-order loops) read and write shared memory with few or no bank conflicts; REV:
+// with bits 10..7 as well, which also spreads the lanes of a bit-reversed order (their index
+// bits are the high ones).  Linear over XOR, so swz(a | b) = swz(a) ^ swz(b) for disjoint bits.
+template <bool REV = false>
+__host__ __device__ constexpr uint32_t swz(uint32_t idx) {
+  return idx ^ ((REV ? (idx >> 4) ^ (idx >> 7) : idx >> 4) & 15u);
+}
 
 // x less 2p unless that is negative.  For coefficients that began in [0, 2p) x stays below 4p
 // < 2^63 and the sign bit tells; ANY: for words of any size (what a decryption may meet) only
@@ -74,21 +78,21 @@ __device__ __forceinline__ void ntt_passes(uint64_t *s, const ulonglong2 *__rest
     if constexpr (!FIRST) __syncthreads();
     for (uint32_t g = threadIdx.x; g < N / 8; g += blockDim.x) {
       const uint32_t base = ((g >> LO) << (LO + 3)) | (g & ((1u << LO) - 1));
-      const uint32_t at = swz(base);
+      const uint32_t at = swz<ANY>(base);
       uint64_t x[8];
       if constexpr (FIRST) {
 #pragma unroll
         for (uint32_t r = 0; r < 8; r++) x[r] = load(base | (r << LO));
       } else {
 #pragma unroll
-        for (uint32_t r = 0; r < 8; r++) x[r] = s[at ^ swz(r << LO)];
+        for (uint32_t r = 0; r < 8; r++) x[r] = s[at ^ swz<ANY>(r << LO)];
       }
       ntt_layer<LOGN, LO, 2, ANY>(x, base, tw, np, p2);
       if constexpr (LO + 1 >= 3) ntt_layer<LOGN, LO, 1, ANY>(x, base, tw, np, p2);
       if constexpr (LO >= 3) ntt_layer<LOGN, LO, 0, ANY>(x, base, tw, np, p2);
       if constexpr (FIRST && ALIAS) __syncthreads();
 #pragma unroll
-      for (uint32_t r = 0; r < 8; r++) s[at ^ swz(r << LO)] = x[r];
+      for (uint32_t r = 0; r < 8; r++) s[at ^ swz<ANY>(r << LO)] = x[r];
     }
     ntt_passes<LOGN, TOP - 3, false, ALIAS, ANY>(s, tw, np, p2, load);
   }
@@ -96,7 +100,7 @@ __device__ __forceinline__ void ntt_passes(uint64_t *s, const ulonglong2 *__rest
 
 // The reference's butterflies with its lazy reductions, so its output bits.  The first pass
 // takes its inputs from load(idx), coefficient idx, in [0, 2p) unless ANY; the output is left
-// in s[swz(idx)] (after a barrier).
+// in s[swz<ANY>(idx)] (after a barrier).
 // 512 <= N <= 8192; any block size, but N/8 threads with ALIAS: load reads memory that s
 // overlaps, so no thread writes s before all have loaded.
 template <int LOGN, bool ALIAS, bool ANY = false, class Load>
@@ -108,7 +112,7 @@ __device__ __forceinline__ void ntt_lazy(uint64_t *s, const ulonglong2 *__restri
   // Bits 2..0 on 8 consecutive coefficients: one layer, then the fused last two.
   const ulonglong2 w1 = __ldg(tw + N - 4 + 1);
   for (uint32_t g = threadIdx.x; g < N / 8; g += blockDim.x) {
-    const uint32_t base = g * 8, at = swz(base);
+    const uint32_t base = g * 8, at = swz<ANY>(base);
     uint64_t x[8];
 #pragma unroll
     for (uint32_t r = 0; r < 8; r++) x[r] = s[at ^ r];

@@ -349,8 +349,6 @@ cudaError_t launch_c(const ReplyLevelArgs &a, const ParamSet &ps, const DevModul
     return cudaErrorInvalidValue;
   using S = Cfg<W, C, E, NS, TB, IPT, GRP>;
   auto kern = reply_tma_kernel<W, C, E, NS, TB, IPT, GRP>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kBytes);
-  if (e != cudaSuccess) return e;
   if (GRP && (a.P != 1 || ((groups + C - 1) / C * C + 1) * a.n_i >= (1ull << 31))) return cudaErrorInvalidValue;
   const uint32_t col_blocks = GRP ? 1 : (uint32_t)((a.P + C - 1) / C);
   const uint64_t blocks = GRP ? (groups + C - 1) / C : groups;
@@ -379,8 +377,6 @@ cudaError_t launch_tasks_c(const uint64_t *const *db, const uint64_t *const *que
   if (e != cudaSuccess) return e;
   using S = Cfg<W, C, E, NS, TB, IPT, GRP>;
   auto kern = reply_tma_tasks_kernel<W, C, E, NS, TB, IPT, GRP>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kBytes);
-  if (e != cudaSuccess) return e;
   if (GRP && (P != 1 || ((groups + C - 1) / C * C + 1) * n_i >= (1ull << 31))) return cudaErrorInvalidValue;
   const uint32_t col_blocks = GRP ? 1 : (uint32_t)((P + C - 1) / C);
   const uint64_t blocks = GRP ? (groups + C - 1) / C : groups;
@@ -400,13 +396,15 @@ struct TileEntry {
   SingleFn single;
   TasksFn tasks;
   const void *single_kernel, *tasks_kernel;
+  size_t bytes;  // dynamic shared memory of both
 };
 
 #define XPIR_TILE_G(W, C, E, NS, TB, IPT, GRP)                                                              \
   {                                                                                                        \
     {W, C, E, NS, TB, IPT, GRP}, &launch_c<W, C, E, NS, TB, IPT, GRP>, &launch_tasks_c<W, C, E, NS, TB, IPT, GRP>, \
         (const void *)&reply_tma_kernel<W, C, E, NS, TB, IPT, GRP>,                                          \
-        (const void *)&reply_tma_tasks_kernel<W, C, E, NS, TB, IPT, GRP>                                     \
+        (const void *)&reply_tma_tasks_kernel<W, C, E, NS, TB, IPT, GRP>,                                    \
+        Cfg<W, C, E, NS, TB, IPT, GRP>::kBytes                                                               \
   }
 #define XPIR_TILE(W, C, E, NS, TB, IPT) XPIR_TILE_G(W, C, E, NS, TB, IPT, false)
 
@@ -591,14 +589,14 @@ cudaError_t launch_reply_level(const ReplyLevelArgs &a, const ParamSet &ps, cons
 }
 
 // Loads every compiled reply kernel on the current device (lazy module loading would
-// otherwise do it, and reserve their device memory, at each one's first launch).
+// otherwise do it, and reserve their device memory, at each one's first launch) and grants
+// it its shared memory, which no launch then has to ask for.
 cudaError_t preload_reply_kernels() {
-  cudaFuncAttributes fa;
-  for (const TileEntry &t : kTiles) {
-    cudaError_t e = cudaFuncGetAttributes(&fa, t.single_kernel);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, t.tasks_kernel);
-    if (e != cudaSuccess) return e;
-  }
+  for (const TileEntry &t : kTiles)
+    for (const void *k : {t.single_kernel, t.tasks_kernel}) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.bytes);
+      if (e != cudaSuccess) return e;
+    }
   return cudaSuccess;
 }
 

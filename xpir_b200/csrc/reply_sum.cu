@@ -416,6 +416,7 @@ struct SumEntry {
   int W, C, E, NS, ctas;  // ctas: resident per SM
   SumFn one, runs;
   const void *kernels[2];
+  size_t bytes;  // their dynamic shared memory
 };
 
 template <int W, int C, int E, int NS, bool ONE, int MINB>
@@ -425,8 +426,6 @@ cudaError_t launch_sum(const ReplyTask &one, const ReplyTask *dev, const SumShap
   const uint64_t blocks = (uint64_t)sh.slices * sh.ntasks * sh.col_blocks * sh.runs;
   if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
   auto kern = reply_sum_kernel<W, C, E, NS, ONE, MINB>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kBytes);
-  if (e != cudaSuccess) return e;
   kern<<<(unsigned)blocks, S::kThreads, S::kBytes, stream>>>(one, dev, sh, dm);
   return cudaGetLastError();
 }
@@ -437,7 +436,7 @@ cudaError_t launch_sum(const ReplyTask &one, const ReplyTask *dev, const SumShap
     {                                                                                               \
       (const void *)reply_sum_kernel<W, C, E, NS, true, MINB>,                                      \
           (const void *)reply_sum_kernel<W, C, E, NS, false, MINB>                                  \
-    }                                                                                               \
+    }, SumCfg<W, C, E, NS>::kBytes                                                                  \
   }
 
 constexpr uint32_t kMaxRuns = 64;
@@ -624,7 +623,8 @@ cudaError_t preload_sum_kernels() {
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, query_range_kernel);
   for (const SumEntry &s : kSums)
     for (const void *k : s.kernels)
-      if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.bytes);
   return e;
 }
 
