@@ -102,7 +102,7 @@ struct xpir_b200_db {
   uint64_t element_bytes = 0;
   // Index in status_host of this database's zero hint (AggSource), 0: none.  Words 0 and p,
   // the import of zero bits, keep the residue sums from deciding a chain, so replies from a
-  // database with all-zero polys run slot by slot at once.  Only a hint: it may be set late
+  // database with kZeroPolys all-zero polys run slot by slot at once.  Only a hint: it may be set late
   // (imports from device memory are asynchronous), and the sums notice by themselves.
   int hint = 0;
   bool zero_polys() const { return hint && ((volatile int *)ctx->status_host)[hint] != 0; }

@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(T, MINB) import_kernel(const AggSource src, co
     stage[w] = v;
     any |= v;
   }
-  if (!__syncthreads_or(any != 0) && threadIdx.x == 0 && c == 0 && src.zero_seen && atomicExch(src.zero_seen, 1) == 0)
+  if (!__syncthreads_or(any != 0) && threadIdx.x == 0 && c == 0 && real == src.alpha && src.zero_seen &&
+      atomicAdd(src.zero_seen, 1) + 1 == kZeroPolys)
     *(volatile int *)src.zero_hint = 1;
 
   // Coefficient k, twisted by phi^k: b <= 56 one chunk per coefficient; b > 56 sub-chunks

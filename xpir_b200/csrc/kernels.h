@@ -22,11 +22,16 @@ struct AggSource {
   uint64_t element_bytes;
   uint64_t element_stride;
   uint32_t alpha;
-  // Optional: *zero_seen (device memory, cleared by the caller) and *zero_hint (host memory)
-  // are set when the bits of some poly, and those next to them, are all zero.
+  // Optional: *zero_seen (device memory, cleared by the caller) counts the polys of full groups
+  // whose bits, and those next to them, are all zero; from kZeroPolys on *zero_hint (host
+  // memory) is set.
   int *zero_seen = nullptr;
   int *zero_hint = nullptr;
 };
+
+// Fewer all-zero polys do not keep the residue sums from deciding a chain, wherever they are:
+// seven in a row raise a run's bound by less than 1.0 p, and of the tail's slots five are left.
+constexpr int kZeroPolys = 8;
 
 // Per-modulus constants the device needs, by value.
 struct DevModuli {

@@ -266,7 +266,9 @@ extern "C" int xpir_b200_generate_query(xpir_b200_ctx *ctx, const uint8_t *prng_
     ctx->launches++;
   }
   uint64_t *target = (uint64_t *)query;
-  if (e == cudaSuccess && !out_on_device) {
+  // The kernel stores pairs of words: a device buffer off a 16-byte boundary gets a copy.
+  const bool staged = !out_on_device || ((uintptr_t)query & 15) != 0;
+  if (e == cudaSuccess && staged) {
     e = pool_allocate(ctx, (void **)&d_out, nq * ct_bytes);
     target = d_out;
   }
@@ -283,7 +285,9 @@ extern "C" int xpir_b200_generate_query(xpir_b200_ctx *ctx, const uint8_t *prng_
     XPIR_BY_DEGREE(ps.log_n, XPIR_ENCRYPT)
     ctx->launches++;
   }
-  if (e == cudaSuccess && !out_on_device) e = cudaMemcpyAsync(query, d_out, nq * ct_bytes, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && staged)
+    e = cudaMemcpyAsync(query, d_out, nq * ct_bytes, out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                        st);
   cudaFreeAsync(d_sk, st);
   cudaFreeAsync(d_sks, st);
   if (d_out) cudaFreeAsync(d_out, st);
