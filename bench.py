@@ -40,13 +40,14 @@ sys.path.insert(0, str(ROOT))
 METRIC = "reply-gen DB GB/s vs HBM peak; batched vs plain queries/s; p50/p99 latency"
 
 # dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes (DB + query +
-# replies) of one first-level reply_tma_kernel launch, per workload, each from one
-# `ncu --set full` capture of a smaller case of the same kernel and tile (traffic grows
-# with the elements: each is one DB row and its share of the query):
-#   memory_bound: 10,000 elements, (995.5 + 3.7) MB / 983.1 MB;
-#   recursive:    262,144 elements (16 groups), (1,823 + 6.7) MB / (1,811.9 + 3.1) MB;
-#   plain:        the full workload (L2 flushed before the launch), (73.8 + 1.7) MB / 73.8 MB.
-REPLY_TRAFFIC_PER_ALGORITHMIC_BYTE = {"memory_bound": 1.0164, "recursive": 1.0081, "plain": 1.0219}
+# replies) of one first-level reply launch (reply_sum_kernel, with reply_finish_kernel where
+# the level is cut into runs), per workload, each from one ncu capture of a smaller case of
+# the same kernel (traffic grows with the elements: each is one DB row and its share of the
+# query):
+#   memory_bound: 8,000 elements, (784.9 + 5.2 + 3.4) MB / 786.5 MB;
+#   recursive:    131,072 elements (256 slots of 32 groups), (856.0 + 25.4) MB / 861.9 MB;
+#   plain:        the full workload, (72.6 + 2.2 + 2.7) MB / 73.8 MB.
+REPLY_TRAFFIC_PER_ALGORITHMIC_BYTE = {"memory_bound": 1.0089, "recursive": 1.0226, "plain": 1.0498}
 
 WORKLOADS = {
     # name: N, m, n levels, alpha, elements, element bytes, chosen index, cpu-sample elements
@@ -427,7 +428,7 @@ def measure_single(args, w: dict, world: int, rank: int, local: int, dist) -> di
             traffic = round(algo_bytes * ratio) if ratio else None
             roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                         "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": traffic,
-                        "kernel": "reply_tma_kernel" + (" (level 1)" if len(n) > 1 else ""),
+                        "kernel": "reply_sum_kernel" + (" (level 1)" if len(n) > 1 else ""),
                         "peak_source": peaks["source"], "algorithmic_bytes_per_launch": algo_bytes,
                         "kernel_ms": round(kern_ms, 4), "kernel_launches_timed": kt["reply_launches"][0]}
             if len(n) > 1:
@@ -632,7 +633,7 @@ def measure_batched(args, w: dict, world: int, rank: int, local: int, dist) -> d
             "batched_over_plain": round(value / plain_qps, 3),
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": None,
-                         "kernel": "reply_tma_tasks_kernel (whole batch)", "peak_source": peaks["source"],
+                         "kernel": "reply_sum_kernel (whole batch)", "peak_source": peaks["source"],
                          "algorithmic_bytes_per_launch": batch_bytes, "kernel_ms": round(batched_ms, 4)},
             "cpu_baseline": cpu,
             "e2e": None,
