@@ -95,10 +95,12 @@ bool build_params(uint32_t N, uint32_t m, uint32_t b, ParamSet *ps, std::vector<
   ps->log_n = ilog2(N);
   ps->m = m;
   ps->b = b;
+  ps->factor8 = true;
   tables->assign((size_t)m * kTableSlots * N, 0);
   for (uint32_t c = 0; c < m; c++) {
     const uint64_t p = kModuli[c];
     if (!shoup_factor_ok(p)) return false;
+    ps->factor8 = ps->factor8 && shoup_factor8_ok(p);
     ModulusConsts &mc = ps->mod[c];
     const ShoupConst sc = make_shoup_const(p);
     mc.p = p;

@@ -42,6 +42,7 @@ struct ParamSet {
   uint32_t log_n = 0;
   uint32_t m = 0;        // number of 60-bit moduli
   uint32_t b = 0;        // bits absorbed per coefficient
+  bool factor8 = false;  // every modulus has the reply kernels' fast Shoup factor (shoup_factor8_ok)
   ModulusConsts mod[kMaxModuli];
 };
 

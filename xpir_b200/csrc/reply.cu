@@ -472,10 +472,8 @@ int sm_count() {
 }  // namespace
 
 bool reply_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_i, uint64_t groups) {
-  for (uint32_t c = 0; c < ps.m; c++)
-    if (!shoup_factor8_ok(ps.mod[c].p)) return false;
   // TMA coordinates are 32-bit signed.
-  return ps.N % 16 == 0 && n_real < (1ull << 31) && groups * n_i + 256 < (1ull << 31);
+  return ps.factor8 && ps.N % 16 == 0 && n_real < (1ull << 31) && groups * n_i + 256 < (1ull << 31);
 }
 
 // One-poly levels with at least four groups (per task) take group columns.  Otherwise
