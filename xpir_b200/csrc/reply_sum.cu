@@ -145,6 +145,8 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
         if (*quit) break;
         if (t % 64 == (uint32_t)NS && *(volatile int *)sh.stop) {
           *quit = 1;
+          *(volatile int *)sh.redo = 1;  // also after a call that failed before it cleared the flag
+          __threadfence_system();
           break;
         }
         if (t >= (uint32_t)NS && !wait_or_quit(empty + st, phase, quit)) break;
