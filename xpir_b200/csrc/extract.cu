@@ -371,10 +371,12 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
   for (uint32_t lvl = d; lvl >= 1 && e == cudaSuccess; lvl--) {
     const uint64_t nbr = extract_count(aggregated_bytes, lvl, bits, N, m);
     uint64_t *res = nullptr, *out = nullptr;
-    // The plaintext (plus slack for the last value's straddling word) is read by the
-    // next level as its ciphertexts: size it for both.
-    uint64_t out_words = nbr * abs_words + 3;
-    if (lvl > 1) out_words = std::max<uint64_t>(out_words, extract_count(aggregated_bytes, lvl - 1, bits, N, m) * ct_words);
+    // The plaintext (plus slack for the last value's straddling word) is read by the next
+    // level as its ciphertexts, or copied to the caller: size it for both.  The count's float
+    // arithmetic can fall a few bytes short of a long element; those bytes are zero.
+    const uint64_t used_words = lvl > 1 ? extract_count(aggregated_bytes, lvl - 1, bits, N, m) * ct_words
+                                        : (aggregated_bytes + 7) / 8;
+    const uint64_t out_words = std::max<uint64_t>(nbr * abs_words + 3, used_words);
     if (nbr > 0x7fffffffull) e = cudaErrorInvalidValue;
     const uint32_t rows = std::max(m - 1, bits > 64 ? 2u : 1u);
     const size_t fused_smem = (size_t)(1 + rows) * N * 8;
@@ -402,6 +404,9 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
         XPIR_BY_DEGREE(ps.log_n, XPIR_EXTRACT)
         ctx->launches++;
       }
+      const uint64_t held = nbr * abs_words * 8;
+      if (e == cudaSuccess && delivered && held < aggregated_bytes)
+        e = cudaMemsetAsync((char *)plaintext + held, 0, aggregated_bytes - held, st);
     } else {
       if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&res, nbr * mN * 8);
       if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&out, out_words * 8);
