@@ -1,6 +1,6 @@
 """Where extraction leaves the element: lengths that the float arithmetic of the ciphertext
 count falls short of (the bytes past the last ciphertext's plaintext are zero, whatever the
-caller's buffer held).  Bytes: no tolerance."""
+caller's buffer held), and buffers that overlap the replies.  Bytes: no tolerance."""
 from __future__ import annotations
 
 import numpy as np
@@ -61,3 +61,27 @@ def test_many_bytes_past_the_last_ciphertext(engine, oracle):
         host = np.full(held + over, 0xA5, dtype=np.uint8)
         ctx.extract(key, 1, b, held + over, ct, host)
         assert np.array_equal(host[:held], short.cpu().numpy()) and not host[held:].any()
+
+
+@pytest.mark.parametrize("N,m,polys", [(2048, 2, 900), (512, 1, 3000)])
+@pytest.mark.parametrize("at", ["start", "middle", "last words"])
+def test_in_place(engine, oracle, N, m, polys, at):
+    """The element over the replies it comes from: every ciphertext is read before any byte
+    is written."""
+    torch = pytest.importorskip("torch")
+    b = oracle.bits_per_coeff(N, m, 20)
+    L = polys * (b * N // 8)
+    assert engine.extract_count(L, 1, b, N, m) == polys
+    key, ct = random_words(15, oracle, N, m), random_words(16, oracle, N, m, polys, 2)
+    want = oracle.extract(ct, key, 1, b, N, m, L)
+    first = {"start": 0, "middle": ct.nbytes // 2, "last words": ct.nbytes - 8}[at]
+    with engine.Context(N, m) as ctx:
+        buf = torch.full((ct.nbytes + L,), 0xA5, dtype=torch.uint8, device="cuda")
+        buf[:ct.nbytes] = torch.from_numpy(ct.view(np.uint8)).cuda()
+        torch.cuda.synchronize()
+        ctx.extract(key, 1, b, L, buf[:ct.nbytes], buf[first:first + L])
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[first:first + L], want)
+        assert np.array_equal(got[:first], ct.view(np.uint8)[:first])
+        assert np.array_equal(got[first + L:ct.nbytes], ct.view(np.uint8)[first + L:])
+        assert (got[max(first + L, ct.nbytes):] == 0xA5).all()

@@ -382,8 +382,10 @@ extern "C" int xpir_b200_extract(xpir_b200_ctx *ctx, const uint64_t *secret_key,
     const size_t fused_smem = (size_t)(1 + rows) * N * 8;
     if (nbr >= kFusedCiphertexts && fused_smem <= kFusedSmem) {
       // Only the words past the plaintext need zeroing, and the last level's plaintext can go
-      // straight to an aligned device buffer.
-      delivered = lvl == 1 && out_on_device && ((uintptr_t)plaintext & 7) == 0;
+      // straight to an aligned device buffer, unless that overlaps the ciphertexts other CTAs
+      // may still be reading (extraction in place).
+      delivered = lvl == 1 && out_on_device && ((uintptr_t)plaintext & 7) == 0 &&
+                  !overlap(level_in, nbr * ct_words * 8, plaintext, aggregated_bytes);
       uint64_t *dst = (uint64_t *)plaintext, limit = aggregated_bytes;
       if (!delivered) {
         if (e == cudaSuccess) e = pool_allocate(ctx, (void **)&out, out_words * 8);

@@ -153,6 +153,12 @@ inline cudaError_t pool_allocate(xpir_b200_ctx *ctx, void **buf, size_t bytes) {
   return e;
 }
 
+// Whether two address ranges share a byte.
+inline bool overlap(const void *a, uint64_t a_bytes, const void *b, uint64_t b_bytes) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + b_bytes && y < x + a_bytes;
+}
+
 // Records a CUDA error as the calling thread's xpir_b200_last_cuda_error().
 void note_cuda_error(cudaError_t e);
 }  // namespace xpir
