@@ -191,6 +191,29 @@ std::vector<uint64_t> plan_key(const xpir_b200_ctx *ctx, const xpir_b200_request
   return key;
 }
 
+// Whether any request's replies lie over a query of the batch.
+bool in_place(const std::vector<Group> &groups, const xpir_b200_request *reqs, uint64_t ct_bytes) {
+  struct Range {
+    uintptr_t from, to;
+  };
+  std::vector<Range> queries;
+  for (const Group &g : groups) {
+    uint64_t total_ct = 0;
+    for (uint32_t lvl = 0; lvl < g.d; lvl++) total_ct += g.n[lvl];
+    for (uint32_t i : g.reqs) queries.push_back({(uintptr_t)reqs[i].query, (uintptr_t)reqs[i].query + total_ct * ct_bytes});
+  }
+  std::sort(queries.begin(), queries.end(), [](const Range &a, const Range &b) { return a.from < b.from; });
+  for (size_t i = 1; i < queries.size(); i++) queries[i].to = std::max(queries[i].to, queries[i - 1].to);
+  for (const Group &g : groups)
+    for (uint32_t i : g.reqs) {
+      const uintptr_t from = (uintptr_t)reqs[i].replies, to = from + g.sh.P[g.d - 1] * ct_bytes;
+      const auto after = std::lower_bound(queries.begin(), queries.end(), to,
+                                          [](const Range &a, uintptr_t end) { return a.from < end; });
+      if (after != queries.begin() && (after - 1)->to > from) return true;
+    }
+  return false;
+}
+
 constexpr size_t kMaxPlans = 8;
 
 }  // namespace
@@ -244,6 +267,8 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   }
   if (groups.empty()) return overall;
   const Sizes z = sizes_of(ctx, groups);
+  // Replies over a query: a repeat would read what they replaced, so no sums from the start.
+  const bool slots = in_place(groups, reqs, ct_bytes);
   ctx->status_host[0] = ctx->status_host[1] = 0;
 
   // Ends the call.  Where residue sums asked for it, the batch first runs once more slot by
@@ -310,7 +335,7 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
     // The pinned table may be rewritten here: the previous call on this context ended
     // with a stream synchronisation, so its copy has completed.
     e = enqueue(ctx, groups, reqs, (uint64_t *)wa, (uint64_t *)wb, (ReplyTask *)ctx->tasks_host,
-                (ReplyTask *)ctx->tasks_dev);
+                (ReplyTask *)ctx->tasks_dev, slots);
     return finish(e, wa, wb, ctx->tasks_host, ctx->tasks_dev);
   }
 
@@ -335,13 +360,13 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   // produces this submission's replies.
   if (e == cudaSuccess)
     e = enqueue(ctx, groups, reqs, (uint64_t *)plan->ws_a, (uint64_t *)plan->ws_b, (ReplyTask *)plan->host_tasks,
-                (ReplyTask *)plan->dev_tasks);
+                (ReplyTask *)plan->dev_tasks, slots);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     const uint64_t before = ctx->launches;
     const cudaError_t ee = enqueue(ctx, groups, reqs, (uint64_t *)plan->ws_a, (uint64_t *)plan->ws_b,
-                                   (ReplyTask *)plan->host_tasks, (ReplyTask *)plan->dev_tasks);
+                                   (ReplyTask *)plan->host_tasks, (ReplyTask *)plan->dev_tasks, slots);
     plan->launches = ctx->launches - before;
     ctx->launches = before;  // captured, not launched
     e = cudaStreamEndCapture(ctx->stream, &plan->graph);

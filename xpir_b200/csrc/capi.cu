@@ -582,7 +582,10 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
     XPIR_TRY(cudaStreamSynchronize(ctx->stream));
     return XPIR_B200_OK;
   };
-  if ((rc = run_levels(db->zero_polys())) != XPIR_B200_OK) return rc;
+  // Replies over the query: a repeat would read what they replaced, so no sums from the start.
+  const bool in_place =
+      query_on_device && out_on_device && overlap(query, total_ct * ct_bytes, replies, final_bytes);
+  if ((rc = run_levels(in_place || db->zero_polys())) != XPIR_B200_OK) return rc;
   if (((volatile int *)ctx->status_host)[1] != 0) {
     XPIR_TRY(cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream));
     if ((rc = run_levels(true)) != XPIR_B200_OK) return rc;

@@ -86,10 +86,11 @@ extern "C" int xpir_b200_reply_noalloc(xpir_b200_ctx *ctx, const xpir_b200_db *d
   using namespace xpir;
   if (!ctx || !db || !n || !query_dev || !replies_dev || d == 0 || d > XPIR_B200_MAX_LEVELS) return XPIR_B200_ERR_ARG;
   if (db->ctx != ctx) return XPIR_B200_ERR_ARG;
-  uint64_t slots = 1;
+  uint64_t slots = 1, total_ct = 0;
   for (uint32_t i = 0; i < d; i++) {
     if (n[i] == 0 || slots > UINT64_MAX / n[i]) return XPIR_B200_ERR_ARG;
     slots *= n[i];
+    total_ct += n[i];
   }
   if (slots < db->n_agg) return XPIR_B200_ERR_ARG;
 
@@ -178,7 +179,9 @@ extern "C" int xpir_b200_reply_noalloc(xpir_b200_ctx *ctx, const xpir_b200_db *d
     }
     return cudaStreamSynchronize(ctx->stream);
   };
-  if ((e = run_levels(db->zero_polys())) != cudaSuccess) return status_of(e);
+  // Replies over the query: a repeat would read what they replaced (as xpir_b200_reply).
+  const bool in_place = overlap(query_dev, total_ct * ct_bytes, replies_dev, final_bytes);
+  if ((e = run_levels(in_place || db->zero_polys())) != cudaSuccess) return status_of(e);
   if (((volatile int *)ctx->status_host)[1] != 0) {
     e = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
     if (e == cudaSuccess) e = run_levels(true);
