@@ -90,12 +90,14 @@ Sizes sizes_of(const xpir_b200_ctx *ctx, const std::vector<Group> &groups) {
 }
 
 // Enqueues every launch of the batch on the context's stream; by_slot: every level with the
-// slot-by-slot kernel (after the residue sums asked for it).
+// slot-by-slot kernel (after the residue sums asked for it).  The redo flags follow the order
+// of the groups and their requests.
 cudaError_t enqueue(xpir_b200_ctx *ctx, const std::vector<Group> &groups, const xpir_b200_request *reqs,
                     uint64_t *ws_a, uint64_t *ws_b, ReplyTask *host_tasks, ReplyTask *dev_tasks,
                     bool by_slot = false) {
   const uint64_t mN = (uint64_t)ctx->ps.m * ctx->ps.N, ct_words = 2 * mN, ct_bytes = ct_words * 8;
   size_t task_off = 0;
+  uint32_t first = 0;  // the group's first request among the redo flags
   for (const Group &g : groups) {
     ParamSet ps = ctx->ps;
     ps.b = g.db->b;
@@ -119,7 +121,7 @@ cudaError_t enqueue(xpir_b200_ctx *ctx, const std::vector<Group> &groups, const 
       const bool sums = !slots && sum_level(ctx, ps, n_real, live, P, g.n[lvl], groups_l, k);
       const uint64_t active = active_groups(sums ? live : n_real, g.n[lvl], groups_l);
       cudaError_t e =
-          sums ? launch_sum_level(sum_args(ctx, n_real, live, P, groups_l, g.n[lvl], last), db.data(), q.data(),
+          sums ? launch_sum_level(sum_args(ctx, n_real, live, P, groups_l, g.n[lvl], last, first), db.data(), q.data(),
                                   out.data(), k, ps, dm, host_tasks + task_off, dev_tasks + task_off, ctx->stream,
                                   &launched)
                : launch_reply_tasks(db.data(), q.data(), out.data(), k, n_real, P, groups_l, g.n[lvl], ps, dm,
@@ -151,6 +153,7 @@ cudaError_t enqueue(xpir_b200_ctx *ctx, const std::vector<Group> &groups, const 
         return e;
       }
     }
+    first += k;
   }
   return cudaSuccess;
 }
@@ -269,19 +272,28 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   const Sizes z = sizes_of(ctx, groups);
   // Replies over a query: a repeat would read what they replaced, so no sums from the start.
   const bool slots = in_place(groups, reqs, ct_bytes);
-  ctx->status_host[0] = ctx->status_host[1] = 0;
+  clear_status(ctx, count);
 
-  // Ends the call.  Where residue sums asked for it, the batch first runs once more slot by
+  // Ends the call.  The queries that residue sums could not decide first run once more slot by
   // slot, in the given workspaces and task tables.
   auto finish = [&](cudaError_t err, void *wa = nullptr, void *wb = nullptr, void *ht = nullptr,
                     void *dt = nullptr) -> int {
     cudaError_t se = cudaStreamSynchronize(ctx->stream);  // also on error: nothing left in flight
     if (err == cudaSuccess) err = se;
-    if (err == cudaSuccess && ((volatile int *)ctx->status_host)[1] != 0) {
-      ctx->status_host[0] = ctx->status_host[1] = 0;
-      err = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
+    std::vector<Group> again;
+    uint64_t place = 0;
+    for (const Group &g : groups) {
+      Group undecided = g;
+      undecided.reqs.clear();
+      for (uint32_t i : g.reqs)
+        if (asked_again(ctx, place++)) undecided.reqs.push_back(i);
+      if (!undecided.reqs.empty()) again.push_back(undecided);
+    }
+    if (err == cudaSuccess && !again.empty()) {
+      clear_status(ctx, count);
+      err = clear_stop(ctx);
       if (err == cudaSuccess)
-        err = enqueue(ctx, groups, reqs, (uint64_t *)wa, (uint64_t *)wb, (ReplyTask *)ht, (ReplyTask *)dt, true);
+        err = enqueue(ctx, again, reqs, (uint64_t *)wa, (uint64_t *)wb, (ReplyTask *)ht, (ReplyTask *)dt, true);
       se = cudaStreamSynchronize(ctx->stream);
       if (err == cudaSuccess) err = se;
     }
@@ -440,7 +452,7 @@ extern "C" int xpir_b200_autotune(xpir_b200_ctx *ctx, const xpir_b200_db *db, ui
       float ms = 0;
       ReplyTask tasks[2];
       for (int rep_i = 0; rep_i < 2 && e == cudaSuccess; rep_i++) {
-        ctx->status_host[1] = 0;
+        clear_status(ctx);
         e = cudaEventRecord(e0, ctx->stream);
         if (e == cudaSuccess)
           e = launch_sum_level(sum_args(ctx, in_real, in_real, sh.P[lvl], sh.groups[lvl], n[lvl], true), &in, &q, &rep,
@@ -449,9 +461,9 @@ extern "C" int xpir_b200_autotune(xpir_b200_ctx *ctx, const xpir_b200_db *db, ui
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
       }
-      if (e == cudaSuccess && ((volatile int *)ctx->status_host)[1] != 0) {
+      if (e == cudaSuccess && asked_again(ctx)) {
         sums = false;  // not decided by sums: the level's replies from a tile again
-        e = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
+        e = clear_stop(ctx);
         if (e == cudaSuccess) e = launch_reply_level(a, ps, dm, ctx->stream, nullptr, ctx->status_dev, best);
       }
       ctx->status_host[1] = 0;

@@ -210,26 +210,26 @@ int xpir_b200_ctx_create(xpir_b200_ctx **out, int device, uint32_t N, uint32_t m
     uint64_t keep = UINT64_MAX;
     rc = cuda_status(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
   }
-  // One allocation: the tables, the zero bit stream's import and the stop flag.
+  // One allocation: the tables, the zero bit stream's import and the stop flags.
   const uint64_t zero_words = (uint64_t)m * N;
   if (rc == XPIR_B200_OK)
-    rc = cuda_status(cudaMalloc(&ctx->d_tables, (tables.size() + zero_words + 2) * sizeof(uint64_t)));
+    rc = cuda_status(cudaMalloc(&ctx->d_tables, (tables.size() + zero_words) * sizeof(uint64_t) + kRedoFlags * sizeof(int)));
   if (rc == XPIR_B200_OK)
     rc = cuda_status(cudaMemcpy(ctx->d_tables, tables.data(), tables.size() * sizeof(uint64_t),
                                 cudaMemcpyHostToDevice));
   if (rc == XPIR_B200_OK) {
     ctx->zero_poly = ctx->d_tables + tables.size();
-    ctx->stop_flag = (int *)(ctx->zero_poly + zero_words);
-    rc = cuda_status(cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream));
+    ctx->stop_flags = (int *)(ctx->zero_poly + zero_words);
+    rc = cuda_status(clear_stop(ctx));
   }
   if (rc == XPIR_B200_OK)
     rc = cuda_status(launch_zero_poly(ctx->ps, make_dev_moduli(ctx->ps), ctx->d_tables, ctx->zero_poly, ctx->stream));
   if (rc == XPIR_B200_OK) rc = cuda_status(take_part(device, &ctx->ws_part));
-  if (rc == XPIR_B200_OK) rc = cuda_status(cudaHostAlloc(&ctx->status_host, (2 + kZeroHints) * sizeof(int),
+  if (rc == XPIR_B200_OK) rc = cuda_status(cudaHostAlloc(&ctx->status_host, (kFirstHint + kZeroHints) * sizeof(int),
                                                          cudaHostAllocMapped));
   if (rc == XPIR_B200_OK) {
-    ctx->status_host[0] = ctx->status_host[1] = 0;
-    for (int i = 1 + kZeroHints; i >= 2; i--) ctx->free_hints.push_back(i);
+    clear_status(ctx, kRedoFlags);
+    for (int i = kFirstHint + kZeroHints - 1; i >= kFirstHint; i--) ctx->free_hints.push_back(i);
     rc = cuda_status(cudaHostGetDevicePointer((void **)&ctx->status_dev, ctx->status_host, 0));
   }
   if (rc != XPIR_B200_OK) {
@@ -532,7 +532,7 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
   auto run_levels = [&](bool by_slot) -> int {
     const uint64_t *in = db->d_polys, *q = dq;
     uint64_t in_real = db->n_agg, in_live = db->n_agg;  // elements past in_live: import of zero bits
-    ctx->status_host[0] = ctx->status_host[1] = 0;
+    clear_status(ctx);
     for (uint32_t lvl = 0; lvl < d; lvl++) {
       const bool last = lvl + 1 == d;
       uint64_t *rep = (last && out_on_device) ? (uint64_t *)replies : (uint64_t *)ctx->ws_a;
@@ -586,8 +586,8 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
   const bool in_place =
       query_on_device && out_on_device && overlap(query, total_ct * ct_bytes, replies, final_bytes);
   if ((rc = run_levels(in_place || db->zero_polys())) != XPIR_B200_OK) return rc;
-  if (((volatile int *)ctx->status_host)[1] != 0) {
-    XPIR_TRY(cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream));
+  if (asked_again(ctx)) {
+    XPIR_TRY(clear_stop(ctx));
     if ((rc = run_levels(true)) != XPIR_B200_OK) return rc;
   }
   for (uint32_t k = 0; k < 2 * d; k++) {

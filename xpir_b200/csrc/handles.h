@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <functional>
 #include <map>
@@ -31,7 +33,7 @@ struct xpir_b200_ctx {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t query_copied = nullptr;
   xpir::ParamSet ps;           // b is set per database
-  uint64_t *d_tables = nullptr;  // also holds zero_poly and stop_flag
+  uint64_t *d_tables = nullptr;  // also holds zero_poly and stop_flags
   std::mutex mu;
   std::atomic<uint64_t> launches{0};  // engine kernels launched (also counted off the lock)
   std::atomic<int> servers{0};         // servers with a lane on this context
@@ -50,8 +52,8 @@ struct xpir_b200_ctx {
   // generation, extraction): it keeps freed memory for the next call (release threshold
   // UINT64_MAX), so that a call after the first maps no new device memory.
   cudaMemPool_t pool = nullptr;
-  // mapped pinned memory: [0] kernel status, [1] redo (SumLevelArgs), then kZeroHints ints
-  // that databases hold one of each (xpir_b200_db::hint)
+  // mapped pinned memory: [0] kernel status, kRedoFlags redo flags (SumLevelArgs), then
+  // kZeroHints ints that databases hold one of each (xpir_b200_db::hint)
   int *status_host = nullptr;
   // The polys of the last freed database (at most kSpareBytes), for the next import: mapping
   // and unmapping 655 MB costs more than importing them.  Released with the context, and when
@@ -60,7 +62,7 @@ struct xpir_b200_ctx {
   size_t spare_bytes = 0;
   int *status_dev = nullptr;
   uint64_t *zero_poly = nullptr;  // [m][N]: import of a zero bit stream
-  int *stop_flag = nullptr;       // SumLevelArgs::stop
+  int *stop_flags = nullptr;      // SumLevelArgs::stop, kRedoFlags ints
   uint64_t *ws_part = nullptr;    // residues of runs (SumLevelArgs::part), kPartWords words
   std::vector<int> free_hints;   // indexes of status_host that no database holds
   std::set<xpir_b200_db *> dbs;  // databases imported through this context
@@ -77,6 +79,7 @@ struct xpir_b200_ctx {
 };
 
 constexpr int kZeroHints = 1022;
+constexpr int kFirstHint = 1 + (int)xpir::kRedoFlags;  // in status_host
 constexpr size_t kSpareBytes = 1ull << 30;
 
 // Workspace of the residue sums' runs: 3.8 MiB per context, taken with it, so that no reply
@@ -116,9 +119,22 @@ inline bool sum_level(const xpir_b200_ctx *ctx, const xpir::ParamSet &ps, uint64
 }
 
 inline xpir::SumLevelArgs sum_args(const xpir_b200_ctx *ctx, uint64_t n_real, uint64_t n_live, uint64_t P,
-                                   uint64_t n_groups, uint64_t n_i, bool write_idle) {
-  return {n_real,       n_live,     P, n_groups, n_i, write_idle, ctx->zero_poly, ctx->ws_part, kPartWords,
-          ctx->status_dev + 1, ctx->status_dev, ctx->stop_flag};
+                                   uint64_t n_groups, uint64_t n_i, bool write_idle, uint32_t first = 0) {
+  return {n_real,     n_live, P, n_groups, n_i, write_idle, ctx->zero_poly, ctx->ws_part, kPartWords,
+          ctx->status_dev + 1, ctx->status_dev, ctx->stop_flags, first};
+}
+
+// Clears the kernel status and the redo flags of a call's queries.
+inline void clear_status(xpir_b200_ctx *ctx, uint64_t queries = 1) {
+  memset(ctx->status_host, 0, (1 + std::min<uint64_t>(queries, xpir::kRedoFlags)) * sizeof(int));
+}
+// Whether query i of the call that ended has to be repeated slot by slot.
+inline bool asked_again(const xpir_b200_ctx *ctx, uint64_t i = 0) {
+  return ((volatile int *)ctx->status_host)[1 + std::min<uint64_t>(i, xpir::kRedoFlags - 1)] != 0;
+}
+// Lets every CTA work again, before such a repeat.
+inline cudaError_t clear_stop(xpir_b200_ctx *ctx) {
+  return cudaMemsetAsync(ctx->stop_flags, 0, xpir::kRedoFlags * sizeof(int), ctx->stream);
 }
 
 struct xpir_b200_request;

@@ -165,10 +165,11 @@ bool reply_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_i, ui
 // One recursion level by residue sums and an exact tail (reply_sum.cu), for `ntasks` queries
 // of the same shape: db[t], query[t], out[t] as in ReplyLevelArgs.  Of the n_real elements
 // only the first n_live are in db; the rest are the constant import of a zero bit stream
-// (zero_poly) and their replies, exactly zero, are written only with write_idle.  A level
-// whose replies cannot be shown to equal the slot-by-slot kernel's sets *redo (a
-// device-visible int that the caller clears): the caller then repeats the call with that
-// kernel.
+// (zero_poly) and their replies, exactly zero, are written only with write_idle.  A query
+// whose replies cannot be shown to equal the slot-by-slot kernel's sets its redo flag
+// (device-visible ints that the caller clears): the caller then repeats that query with that
+// kernel.  The flag of task t is redo[min(first + t, kRedoFlags - 1)].
+constexpr uint32_t kRedoFlags = 1024;
 struct SumLevelArgs {
   uint64_t n_real, n_live, P, n_groups, n_i;
   bool write_idle;
@@ -176,7 +177,8 @@ struct SumLevelArgs {
   uint64_t *part;       // workspace of part_words words
   uint64_t part_words;
   int *redo, *status;
-  int *stop;  // device memory: set with *redo, cleared by the caller before it repeats the call
+  int *stop;       // device memory: set with the redo flags, cleared by the caller before it repeats
+  uint32_t first;  // task 0's place among the call's queries
 };
 // Whether a level of this shape takes that path.
 bool sum_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_live, uint64_t P, uint64_t n_i,

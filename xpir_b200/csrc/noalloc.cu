@@ -140,7 +140,7 @@ extern "C" int xpir_b200_reply_noalloc(xpir_b200_ctx *ctx, const xpir_b200_db *d
     const uint64_t *in = db->d_polys;
     const uint64_t *q = (const uint64_t *)query_dev;
     uint64_t in_real = db->n_agg, in_live = db->n_agg;
-    ctx->status_host[0] = ctx->status_host[1] = 0;
+    clear_status(ctx);
     for (uint32_t lvl = 0; lvl < d; lvl++) {
       const bool last = lvl + 1 == d;
       uint64_t *rep = last ? (uint64_t *)replies_dev : (uint64_t *)scratch;
@@ -182,8 +182,8 @@ extern "C" int xpir_b200_reply_noalloc(xpir_b200_ctx *ctx, const xpir_b200_db *d
   // Replies over the query: a repeat would read what they replaced (as xpir_b200_reply).
   const bool in_place = overlap(query_dev, total_ct * ct_bytes, replies_dev, final_bytes);
   if ((e = run_levels(in_place || db->zero_polys())) != cudaSuccess) return status_of(e);
-  if (((volatile int *)ctx->status_host)[1] != 0) {
-    e = cudaMemsetAsync(ctx->stop_flag, 0, sizeof(int), ctx->stream);
+  if (asked_again(ctx)) {
+    e = clear_stop(ctx);
     if (e == cudaSuccess) e = run_levels(true);
     if (e != cudaSuccess) return status_of(e);
   }

@@ -23,8 +23,9 @@
 // kernel spends 56 on a Shoup factor and a Shoup product alone.  1,048,576 x 256 B in 16s:
 // level 1 2.47 -> 1.45 ms.  Up to four columns per CTA share the query words' preparation.
 //
-// What the sums cannot decide sets *redo, and the caller repeats the call slot by slot.  A
-// CTA that finds such a word stops at once, so a query of unreduced words costs one tile.
+// What the sums cannot decide sets the query's redo flag, and the caller repeats that query
+// slot by slot.  A CTA that finds such a word stops at once, and the query's other CTAs that
+// see it, so a query of unreduced words costs one tile.  The other queries go on.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -54,8 +55,13 @@ struct SumShape {
   const uint64_t *zero_poly;  // [m][N] that constant
   uint64_t *part;     // [task][column][half][run][m][N]
   int *redo, *status;
-  int *stop;          // device copy of *redo: CTAs that see it set do no more work
+  int *stop;          // device copy of redo: a query's CTAs that see its flag set do no more work
+  uint32_t first;     // task 0's place among the flags
 };
+
+__host__ __device__ __forceinline__ uint32_t flag_of(uint32_t first, uint32_t task) {
+  return first + task < kRedoFlags ? first + task : kRedoFlags - 1;
+}
 
 template <int W, int C, int E, int NS>
 struct SumCfg {
@@ -143,9 +149,9 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
       uint32_t t = 0, st = 0, phase = 1;
       for (; t < tiles; ++t) {
         if (*quit) break;
-        if (t % 64 == (uint32_t)NS && *(volatile int *)sh.stop) {
+        if (t % 64 == (uint32_t)NS && *(volatile int *)(sh.stop + flag_of(sh.first, task_id))) {
           *quit = 1;
-          *(volatile int *)sh.redo = 1;  // also after a call that failed before it cleared the flag
+          *(volatile int *)(sh.redo + flag_of(sh.first, task_id)) = 1;  // also after a call that failed before it cleared the flag
           __threadfence_system();
           break;
         }
@@ -299,8 +305,8 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
   }
   if (bad) {
     *quit = 1;
-    *(volatile int *)sh.stop = 1;
-    *(volatile int *)sh.redo = 1;
+    *(volatile int *)(sh.stop + flag_of(sh.first, task_id)) = 1;
+    *(volatile int *)(sh.redo + flag_of(sh.first, task_id)) = 1;
   }
   if (late && !*quit) *(volatile int *)sh.status = kStatusWaitTimeout;
   if (bad || late) __threadfence_system();
@@ -388,7 +394,7 @@ __device__ __forceinline__ void finish_tile(const ReplyTask &task, const SumShap
     task.out[(j * 2 + w) * mN + at0 + k] = zero_steps(s.rop, (zero_p ? 0 : sh.idle) + sh.pad, p);
   }
   if (bad) {
-    *(volatile int *)sh.redo = 1;
+    *(volatile int *)(sh.redo + flag_of(sh.first, blockIdx.z)) = 1;
     __threadfence_system();
   }
 }
@@ -541,6 +547,7 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
   sh.redo = a.redo;
   sh.status = a.status;
   sh.stop = a.stop;
+  sh.first = a.first;
   // Elements past n_live (idle): the group that holds the first of them is a launch of its
   // own when there are others, since its chain ends at another slot.
   const bool idle = a.n_live < a.n_real;
@@ -554,7 +561,7 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
     for (uint32_t t = 0; t < ntasks && pairs; t++) {
       const unsigned blocks = (unsigned)std::min<uint64_t>((pairs + 1023) / 1024, 8ull * sum_sm_count());
       query_range_kernel<<<blocks, 256, 0, stream>>>((const ulonglong2 *)(query[t] + from * ct_words), pairs, ps.N,
-                                                     ps.m, dm, a.redo);
+                                                     ps.m, dm, a.redo + flag_of(a.first, t));
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       if (launches) (*launches)++;
