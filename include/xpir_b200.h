@@ -85,8 +85,8 @@ XPIR_B200_API int xpir_b200_ctx_stream(xpir_b200_ctx *ctx, void **stream);
 XPIR_B200_API int xpir_b200_ctx_synchronize(xpir_b200_ctx *ctx);
 /* Number of engine kernels launched on this context so far. */
 XPIR_B200_API int xpir_b200_ctx_launch_count(xpir_b200_ctx *ctx, uint64_t *count);
-/* Test support for the reply kernel's bounded waits; no counterpart in the reference.
- * Every wait in the reply kernel gives up after a fixed number of polls (about 2.6 s),
+/* Test support for the reply kernels' bounded waits; no counterpart in the reference.
+ * Every wait in the reply kernels gives up after a fixed number of polls (about 2.6 s),
  * records the failure and lets the kernel return, so that a stalled pipeline ends in
  * XPIR_B200_ERR_TIMEOUT instead of a hang.  For the following xpir_b200_reply calls on
  * this context: spin_limit > 0 shortens the limit of the consumers' waits and of the copy

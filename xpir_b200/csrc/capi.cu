@@ -544,8 +544,9 @@ int xpir_b200_reply(xpir_b200_ctx *ctx, const xpir_b200_db *db, uint32_t d, cons
       cudaError_t le;
       if (sums) {
         ReplyTask tasks[2];
-        le = launch_sum_level(sum_args(ctx, in_real, in_live, Ps[lvl], groups[lvl], n[lvl], last), &in, &q, &rep, 1, ps,
-                              dm, tasks, nullptr, ctx->stream, &launched);
+        SumLevelArgs a = sum_args(ctx, in_real, in_live, Ps[lvl], groups[lvl], n[lvl], last);
+        a.wait_test = ctx->wait_test;
+        le = launch_sum_level(a, &in, &q, &rep, 1, ps, dm, tasks, nullptr, ctx->stream, &launched);
       } else {
         ReplyLevelArgs a{in, in_real, Ps[lvl], groups[lvl], n[lvl], q, rep};
         a.write_idle = last;

@@ -111,17 +111,16 @@ struct xpir_b200_db {
   bool zero_polys() const { return hint && ((volatile int *)ctx->status_host)[hint] != 0; }
 };
 
-// Whether a level takes the residue-sum path: no pinned or tuned tile shape, no wait test.
+// Whether a level takes the residue-sum path: no pinned or tuned tile shape.
 inline bool sum_level(const xpir_b200_ctx *ctx, const xpir::ParamSet &ps, uint64_t n_real, uint64_t n_live, uint64_t P,
                       uint64_t n_i, uint64_t groups, uint64_t ntasks) {
-  return ctx->wait_test.spin_limit == 0 && ctx->wait_test.withhold_tile < 0 &&
-         tuned_tile(ctx, P, n_i, groups) < 0 && xpir::sum_level_supported(ps, n_real, n_live, P, n_i, groups, ntasks);
+  return tuned_tile(ctx, P, n_i, groups) < 0 && xpir::sum_level_supported(ps, n_real, n_live, P, n_i, groups, ntasks);
 }
 
 inline xpir::SumLevelArgs sum_args(const xpir_b200_ctx *ctx, uint64_t n_real, uint64_t n_live, uint64_t P,
                                    uint64_t n_groups, uint64_t n_i, bool write_idle, uint32_t first = 0) {
   return {n_real,     n_live, P, n_groups, n_i, write_idle, ctx->zero_poly, ctx->ws_part, kPartWords,
-          ctx->status_dev + 1, ctx->status_dev, ctx->stop_flags, first};
+          ctx->status_dev, ctx->stop_flags, first, {}};
 }
 
 // Clears the kernel status and the redo flags of a call's queries.

@@ -81,7 +81,7 @@ cudaError_t launch_import(const AggSource &src, uint64_t groups, uint64_t P, con
                           const DevModuli &dm, const uint64_t *tables, uint64_t *out, cudaStream_t stream,
                           const ImportRows *rows = nullptr, uint32_t *launches = nullptr);
 
-// Test support for the reply kernel's bounded waits (xpir_b200_ctx_set_wait_test): a
+// Test support for the reply kernels' bounded waits (xpir_b200_ctx_set_wait_test): a
 // shorter limit for the waits of the consumer warps and of the copy producer's ring, and
 // a tile whose copies the producer never issues (-1: none), so that the waits for that
 // tile run out, the kernel records kStatusWaitTimeout and returns.  The producer's final
@@ -168,7 +168,7 @@ bool reply_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_i, ui
 // (zero_poly) and their replies, exactly zero, are written only with write_idle.  A query
 // whose replies cannot be shown to equal the slot-by-slot kernel's sets its redo flag
 // (device-visible ints that the caller clears): the caller then repeats that query with that
-// kernel.  The flag of task t is redo[min(first + t, kRedoFlags - 1)].
+// kernel.  The flag of task t is status[1 + min(first + t, kRedoFlags - 1)].
 constexpr uint32_t kRedoFlags = 1024;
 struct SumLevelArgs {
   uint64_t n_real, n_live, P, n_groups, n_i;
@@ -176,9 +176,10 @@ struct SumLevelArgs {
   const uint64_t *zero_poly;
   uint64_t *part;       // workspace of part_words words
   uint64_t part_words;
-  int *redo, *status;
+  int *status;     // the kernel status, then the redo flags
   int *stop;       // device memory: set with the redo flags, cleared by the caller before it repeats
   uint32_t first;  // task 0's place among the call's queries
+  WaitTest wait_test;
 };
 // Whether a level of this shape takes that path.
 bool sum_level_supported(const ParamSet &ps, uint64_t n_real, uint64_t n_live, uint64_t P, uint64_t n_i,

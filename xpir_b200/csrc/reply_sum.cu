@@ -42,6 +42,7 @@ namespace {
 
 constexpr uint32_t kTopOfP = 0x1fffffffu;  // p >> 32 of every modulus
 
+// A kernel parameter: kept small (16 bytes more took the 1,000 x 12 KB reply from 38.7 to 39.2 us).
 struct SumShape {
   uint64_t P, n_i;
   uint64_t cols;      // groups with live elements * P
@@ -51,31 +52,42 @@ struct SumShape {
   uint32_t col_blocks, ntasks, runs;
   uint32_t n_eff;     // slots with live elements (of a full group)
   uint32_t prefix;    // slots summed; the exact tail takes the rest
-  uint64_t idle, pad;  // slots after n_eff: constant import of a zero bit stream, zero words
+  uint32_t idle, pad;  // slots after n_eff: constant import of a zero bit stream, zero words
   const uint64_t *zero_poly;  // [m][N] that constant
   uint64_t *part;     // [task][column][half][run][m][N]
-  int *redo, *status;
-  int *stop;          // device copy of redo: a query's CTAs that see its flag set do no more work
+  int *status;        // the redo flags follow it
+  int *stop;          // device copies of those: a query's CTAs that see its flag set do no more work
   uint32_t first;     // task 0's place among the flags
+  uint32_t spin_limit;   // polls of a wait
+  uint32_t issued_tiles; // tiles the producer issues at most (test support: it starves the consumers)
 };
 
 __host__ __device__ __forceinline__ uint32_t flag_of(uint32_t first, uint32_t task) {
   return first + task < kRedoFlags ? first + task : kRedoFlags - 1;
 }
 
+// What a CTA rarely needs, in shared memory instead of registers: the products of four
+// columns leave none over.
+struct alignas(16) CtaState {
+  int quit;       // set: the CTA has given up
+  uint32_t flag;  // its query's place among the flags
+};
+
 template <int W, int C, int E, int NS>
 struct SumCfg {
   static constexpr int kThreads = W + 32;
   static constexpr int kX = C * E * W, kQ = E * 2 * W;  // words per stage
-  static constexpr size_t kBytes = (size_t)NS * (kX + kQ) * 8 + 2 * NS * 8 + 16;
+  static constexpr size_t kBytes = (size_t)NS * (kX + kQ) * 8 + 2 * NS * 8 + sizeof(CtaState);
   static_assert(E % 4 == 0 && W % 32 == 0 && W <= 256, "tile shape");
 };
 
-// Waits for a phase; false after the poll limit or when the CTA has given up (*quit).
-__device__ __forceinline__ bool wait_or_quit(uint64_t *bar, uint32_t parity, volatile int *quit) {
-  for (uint32_t i = 0; i < kSpinLimit; ++i) {
+// Waits for a phase; false after `limit` polls or when the CTA has given up.  Not inlined: with
+// the limit a variable, the loop beside the products cost 1 % (1,048,576 x 256 B 1,807 us; as a
+// call 1,793, with the limit a constant 1,792).
+__device__ __noinline__ bool wait_or_quit(uint64_t *bar, uint32_t parity, volatile CtaState *state, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (*quit) return false;
+    if (state->quit) return false;
   }
   return false;
 }
@@ -111,7 +123,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
   uint64_t *xs = sm;                 // [NS][C][E][W]
   uint64_t *qs = xs + NS * S::kX;    // [NS][E][2][W]
   uint64_t *full = qs + NS * S::kQ, *empty = full + NS;
-  volatile int *quit = (volatile int *)(empty + NS);
+  volatile CtaState *state = (volatile CtaState *)(empty + NS);
 
   const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t per_mod = sh.N / W;
@@ -125,7 +137,8 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
 
   if constexpr (!ONE) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (threadIdx.x == 0) {
-    *quit = 0;
+    state->quit = 0;
+    state->flag = flag_of(sh.first, task_id);
     for (int s = 0; s < NS; s++) {
       mbar_init(full + s, 1);
       mbar_init(empty + s, W / 32);
@@ -147,15 +160,15 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
         poly[i] = (int)(j - g * sh.P);
       }
       uint32_t t = 0, st = 0, phase = 1;
-      for (; t < tiles; ++t) {
-        if (*quit) break;
-        if (t % 64 == (uint32_t)NS && *(volatile int *)(sh.stop + flag_of(sh.first, task_id))) {
-          *quit = 1;
-          *(volatile int *)(sh.redo + flag_of(sh.first, task_id)) = 1;  // also after a call that failed before it cleared the flag
+      for (const uint32_t issued = min(tiles, sh.issued_tiles); t < issued; ++t) {
+        if (state->quit) break;
+        if (t % 64 == (uint32_t)NS && *(volatile int *)(sh.stop + state->flag)) {
+          state->quit = 1;
+          *(volatile int *)(sh.status + 1 + state->flag) = 1;  // also after a call that failed before it cleared the flag
           __threadfence_system();
           break;
         }
-        if (t >= (uint32_t)NS && !wait_or_quit(empty + st, phase, quit)) break;
+        if (t >= (uint32_t)NS && !wait_or_quit(empty + st, phase, state, sh.spin_limit)) break;
         mbar_arrive_expect_tx(full + st, (uint32_t)((S::kX + S::kQ) * 8));
         const int slot = (int)(s0 + t * E);
 #pragma unroll
@@ -187,7 +200,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
   uint32_t t = 0, st = 0, phase = 0;
   // Waits for tile t; false (in the whole warp) when it must stop.
   auto tile_ready = [&]() -> bool {
-    const bool ok = mbar_try_wait(full + st, phase) || wait_or_quit(full + st, phase, quit);
+    const bool ok = mbar_try_wait(full + st, phase) || wait_or_quit(full + st, phase, state, sh.spin_limit);
     if (!__any_sync(~0u, bad || !ok)) return true;
     late = !__all_sync(~0u, ok);
     bad = __any_sync(~0u, bad);
@@ -289,7 +302,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
             if (tail[h][i].above)
               bad |= !chain_again(task, sh, j, h, c, at, sum_residue(acc[h][i], p, np, delta), p, np, delta, &rop);
           }
-          task.out[(j * 2 + h) * mN + at] = zero_steps(rop, (zero_p ? 0 : sh.idle) + sh.pad, p);
+          task.out[(j * 2 + h) * mN + at] = zero_steps(rop, (uint64_t)(zero_p ? 0 : sh.idle) + sh.pad, p);
         }
     }
   } else if (!bad && !late) {
@@ -304,11 +317,11 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
       }
   }
   if (bad) {
-    *quit = 1;
-    *(volatile int *)(sh.stop + flag_of(sh.first, task_id)) = 1;
-    *(volatile int *)(sh.redo + flag_of(sh.first, task_id)) = 1;
+    state->quit = 1;
+    *(volatile int *)(sh.stop + state->flag) = 1;
+    *(volatile int *)(sh.status + 1 + state->flag) = 1;
   }
-  if (late && !*quit) *(volatile int *)sh.status = kStatusWaitTimeout;
+  if (late && !state->quit) *(volatile int *)sh.status = kStatusWaitTimeout;
   if (bad || late) __threadfence_system();
 }
 
@@ -391,10 +404,10 @@ __device__ __forceinline__ void finish_tile(const ReplyTask &task, const SumShap
     bad |= !tail_in_range(s, kRunAbove);
     if (s.above) bad |= !chain_again(task, sh, j, w, c, at0 + k, r, p, np, delta, &s.rop);
     const bool zero_p = sh.idle && sh.zero_poly[at0 + k] != 0;
-    task.out[(j * 2 + w) * mN + at0 + k] = zero_steps(s.rop, (zero_p ? 0 : sh.idle) + sh.pad, p);
+    task.out[(j * 2 + w) * mN + at0 + k] = zero_steps(s.rop, (uint64_t)(zero_p ? 0 : sh.idle) + sh.pad, p);
   }
   if (bad) {
-    *(volatile int *)(sh.redo + flag_of(sh.first, blockIdx.z)) = 1;
+    *(volatile int *)(sh.status + 1 + flag_of(sh.first, blockIdx.z)) = 1;
     __threadfence_system();
   }
 }
@@ -544,10 +557,11 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
   sh.ntasks = ntasks;
   sh.zero_poly = a.zero_poly;
   sh.part = a.part;
-  sh.redo = a.redo;
   sh.status = a.status;
   sh.stop = a.stop;
   sh.first = a.first;
+  sh.spin_limit = a.wait_test.spin_limit ? a.wait_test.spin_limit : kSpinLimit;
+  sh.issued_tiles = (uint32_t)a.wait_test.withhold_tile;  // -1: all
   // Elements past n_live (idle): the group that holds the first of them is a launch of its
   // own when there are others, since its chain ends at another slot.
   const bool idle = a.n_live < a.n_real;
@@ -561,7 +575,7 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
     for (uint32_t t = 0; t < ntasks && pairs; t++) {
       const unsigned blocks = (unsigned)std::min<uint64_t>((pairs + 1023) / 1024, 8ull * sum_sm_count());
       query_range_kernel<<<blocks, 256, 0, stream>>>((const ulonglong2 *)(query[t] + from * ct_words), pairs, ps.N,
-                                                     ps.m, dm, a.redo + flag_of(a.first, t));
+                                                     ps.m, dm, a.status + 1 + flag_of(a.first, t));
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       if (launches) (*launches)++;
@@ -575,8 +589,8 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
     sh.n_live = live;
     sh.n_eff = (uint32_t)std::min(a.n_i, live);
     const uint64_t last_real = groups == 1 ? std::min(a.n_i, real) : a.n_i;
-    sh.idle = last_real - sh.n_eff;
-    sh.pad = a.n_i - last_real;
+    sh.idle = (uint32_t)(last_real - sh.n_eff);  // n_i < 2^31 (reply_level_supported)
+    sh.pad = (uint32_t)(a.n_i - last_real);
     const SumEntry &entry = sum_entry((uint32_t)mN, sh.cols, sh.n_eff, ntasks);
     sh.slices = (uint32_t)(mN / entry.W);
     sh.col_blocks = (uint32_t)((sh.cols + entry.C - 1) / entry.C);
