@@ -119,8 +119,10 @@ XPIR_B200_API int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, 
                         uint64_t element_stride, uint32_t alpha, uint32_t bits_per_coeff, int src_on_device,
                         xpir_b200_db **db);
 /* Frees the device copy: the role of imported_database::~imported_database
- * (pir/libpir.cpp:5-11).  The context keeps the memory of one freed database of at most
- * 1 GiB for its next import, and gives it back when it is destroyed or short of memory. */
+ * (pir/libpir.cpp:5-11).  The context keeps the memory of one freed database for the
+ * next import on the device (at most 1 GiB per device over all contexts) and gives it back
+ * when it is destroyed, or when an allocation of any context or server on the device would
+ * fail.  Other allocators in the process do not see it as free until then. */
 XPIR_B200_API int xpir_b200_db_free(xpir_b200_db *db);
 /* Aggregated elements, polys per element, bits per coefficient and HBM bytes held. */
 XPIR_B200_API int xpir_b200_db_info(const xpir_b200_db *db, uint64_t *nb_aggregated, uint64_t *polys_per_element,

@@ -339,7 +339,7 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
       ctx->tasks_dev = ctx->tasks_host = nullptr;
       ctx->tasks_cap = 0;
       const size_t cap = std::max<size_t>(z.tasks, 64);
-      e = cudaMalloc(&ctx->tasks_dev, cap * sizeof(ReplyTask));
+      e = allocate(ctx, &ctx->tasks_dev, cap * sizeof(ReplyTask));
       if (e == cudaSuccess) e = cudaMallocHost(&ctx->tasks_host, cap * sizeof(ReplyTask));
       if (e != cudaSuccess) return finish(e);
       ctx->tasks_cap = cap;
@@ -366,7 +366,7 @@ int xpir::reply_batch_impl(xpir_b200_ctx *ctx, xpir_b200_request *reqs, uint32_t
   if (e == cudaSuccess) e = allocate(ctx, &plan->ws_b, std::max<size_t>(z.ws_b, 256));
   // Two tables: the graph copies the first from host_tasks at every replay, so a repeat of the
   // batch slot by slot fills the second.
-  if (e == cudaSuccess) e = cudaMalloc(&plan->dev_tasks, 2 * z.tasks * sizeof(ReplyTask));
+  if (e == cudaSuccess) e = allocate(ctx, &plan->dev_tasks, 2 * z.tasks * sizeof(ReplyTask));
   if (e == cudaSuccess) e = cudaMallocHost(&plan->host_tasks, 2 * z.tasks * sizeof(ReplyTask));
   // One eager run first: it sets the kernels' attributes outside the capture and
   // produces this submission's replies.
@@ -543,8 +543,8 @@ extern "C" int xpir_b200_measure_costs(xpir_b200_ctx *ctx, uint32_t security_bit
       xpir_b200_db_info(db, &nagg, &P, &bb, &dev);
       replies.assign(P * 2 * m * N, 0);
       void *dq = nullptr, *dr = nullptr;
-      e = cudaMalloc(&dq, query.size() * 8);
-      if (e == cudaSuccess) e = cudaMalloc(&dr, replies.size() * 8);
+      e = allocate(ctx, &dq, query.size() * 8);
+      if (e == cudaSuccess) e = allocate(ctx, &dr, replies.size() * 8);
       if (e == cudaSuccess) e = cudaMemcpy(dq, query.data(), query.size() * 8, cudaMemcpyHostToDevice);
       uint64_t cnt = 0;
       for (int rep = 0; rep < 3 && e == cudaSuccess && rc == XPIR_B200_OK; rep++) {  // warm-up, then timed

@@ -7,7 +7,9 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
+#include <new>
 #include <set>
 #include <vector>
 
@@ -38,7 +40,7 @@ int cuda_status(cudaError_t e) {
     if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
-int grow(xpir_b200_ctx *ctx, void **buf, size_t *have, size_t need) {
+int grow(const xpir_b200_ctx *ctx, void **buf, size_t *have, size_t need) {
   if (need <= *have) return XPIR_B200_OK;
   if (*buf) {
     XPIR_TRY(cudaFree(*buf));
@@ -99,7 +101,7 @@ cudaError_t take_part(int device, uint64_t **out) {
         return cudaSuccess;
       }
   uint64_t *base = nullptr;
-  const cudaError_t e = cudaMalloc(&base, kSlabParts * kPartWords * sizeof(uint64_t));
+  const cudaError_t e = allocate(device, (void **)&base, kSlabParts * kPartWords * sizeof(uint64_t));
   if (e != cudaSuccess) return e;
   g_slabs.push_back({device, base, 1});
   *out = base;
@@ -120,7 +122,95 @@ void give_part(uint64_t *part) {
   }
 }
 
+struct Spare {
+  const xpir_b200_ctx *ctx;
+  int device;
+  void *ptr;
+  size_t bytes;
+};
+std::mutex g_spare_mu;
+std::vector<Spare> g_spares;  // at most one by each context, in the order they were freed
+
+// Frees the spare blocks that `which` picks; whether there were any.
+template <class Which>
+bool free_spares(Which which) {
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  const size_t before = g_spares.size();
+  g_spares.erase(std::remove_if(g_spares.begin(), g_spares.end(),
+                                [&](const Spare &s) {
+                                  if (!which(s)) return false;
+                                  cudaFree(s.ptr);
+                                  return true;
+                                }),
+                 g_spares.end());
+  return g_spares.size() < before;
+}
+
+// `alloc`, and once more without the device's spare blocks when memory is short.
+template <class Alloc>
+cudaError_t with_spares(int device, Alloc alloc) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation && free_spares([&](const Spare &s) { return s.device == device; })) {
+    (void)cudaGetLastError();
+    e = alloc();
+  }
+  return e;
+}
+
 }  // namespace
+
+bool xpir::take_spare(const xpir_b200_ctx *ctx, size_t bytes, void **ptr, size_t *have) {
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  for (auto s = g_spares.begin(); s != g_spares.end(); ++s)
+    if (s->device == ctx->device && bytes <= s->bytes && bytes >= s->bytes / 2) {
+      *ptr = s->ptr;
+      *have = s->bytes;
+      g_spares.erase(s);
+      return true;
+    }
+  return false;
+}
+
+void xpir::keep_spare(const xpir_b200_ctx *ctx, void *ptr, size_t bytes) {
+  bool larger = bytes <= kSpareBytes;  // than what the context keeps already
+  {
+    std::lock_guard<std::mutex> lock(g_spare_mu);
+    for (const Spare &s : g_spares) larger = larger && !(s.ctx == ctx && s.bytes >= bytes);
+  }
+  if (!larger) {
+    cudaFree(ptr);
+    return;
+  }
+  drop_spare(ctx);
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  try {
+    g_spares.push_back({ctx, ctx->device, ptr, bytes});
+  } catch (const std::bad_alloc &) {
+    cudaFree(ptr);
+    return;
+  }
+  size_t total = 0;  // of the device, from the last one back
+  for (size_t i = g_spares.size(); i-- > 0;) {
+    if (g_spares[i].device != ctx->device) continue;
+    total += g_spares[i].bytes;
+    if (total <= kSpareBytes) continue;
+    cudaFree(g_spares[i].ptr);
+    total -= g_spares[i].bytes;
+    g_spares.erase(g_spares.begin() + i);
+  }
+}
+
+void xpir::drop_spare(const xpir_b200_ctx *ctx) {
+  free_spares([&](const Spare &s) { return s.ctx == ctx; });
+}
+
+cudaError_t xpir::allocate(int device, void **buf, size_t bytes) {
+  return with_spares(device, [&] { return cudaMalloc(buf, bytes); });
+}
+
+cudaError_t xpir::pool_allocate(int device, void **buf, size_t bytes, cudaMemPool_t pool, cudaStream_t stream) {
+  return with_spares(device, [&] { return cudaMallocFromPoolAsync(buf, bytes, pool, stream); });
+}
 
 void xpir::note_cuda_error(cudaError_t e) {
   if (e != cudaSuccess) g_last_cuda = e;
@@ -213,7 +303,8 @@ int xpir_b200_ctx_create(xpir_b200_ctx **out, int device, uint32_t N, uint32_t m
   // One allocation: the tables, the zero bit stream's import and the stop flags.
   const uint64_t zero_words = (uint64_t)m * N;
   if (rc == XPIR_B200_OK)
-    rc = cuda_status(cudaMalloc(&ctx->d_tables, (tables.size() + zero_words) * sizeof(uint64_t) + kRedoFlags * sizeof(int)));
+    rc = cuda_status(allocate(ctx, (void **)&ctx->d_tables,
+                              (tables.size() + zero_words) * sizeof(uint64_t) + kRedoFlags * sizeof(int)));
   if (rc == XPIR_B200_OK)
     rc = cuda_status(cudaMemcpy(ctx->d_tables, tables.data(), tables.size() * sizeof(uint64_t),
                                 cudaMemcpyHostToDevice));
@@ -359,14 +450,8 @@ int xpir_b200_db_import(xpir_b200_ctx *ctx, const void *elements, uint64_t nb_el
   db->element_bytes = element_bytes;
   db->alloc_bytes = (words + 2) * sizeof(uint64_t);  // the last two: zero_seen
   cudaError_t e = cudaSuccess;
-  if (ctx->spare && db->alloc_bytes <= ctx->spare_bytes && db->alloc_bytes >= ctx->spare_bytes / 2) {
-    db->d_polys = (uint64_t *)ctx->spare;
-    db->alloc_bytes = ctx->spare_bytes;
-    ctx->spare = nullptr;
-    ctx->spare_bytes = 0;
-  } else {
+  if (!take_spare(ctx, db->alloc_bytes, (void **)&db->d_polys, &db->alloc_bytes))
     e = allocate(ctx, (void **)&db->d_polys, db->alloc_bytes);
-  }
   if (e != cudaSuccess) {
     delete db;
     return cuda_status(e);
@@ -416,13 +501,7 @@ int xpir_b200_db_free(xpir_b200_db *db) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   drop_plans_of(ctx, db->id);
-  if (db->alloc_bytes <= kSpareBytes && db->alloc_bytes > ctx->spare_bytes) {
-    drop_spare(ctx);
-    ctx->spare = db->d_polys;
-    ctx->spare_bytes = db->alloc_bytes;
-  } else {
-    cudaFree(db->d_polys);
-  }
+  keep_spare(ctx, db->d_polys, db->alloc_bytes);
   if (db->hint) ctx->free_hints.push_back(db->hint);
   delete db;
   return XPIR_B200_OK;

@@ -55,11 +55,6 @@ struct xpir_b200_ctx {
   // mapped pinned memory: [0] kernel status, kRedoFlags redo flags (SumLevelArgs), then
   // kZeroHints ints that databases hold one of each (xpir_b200_db::hint)
   int *status_host = nullptr;
-  // The polys of the last freed database (at most kSpareBytes), for the next import: mapping
-  // and unmapping 655 MB costs more than importing them.  Released with the context, and when
-  // an allocation of this context fails.
-  void *spare = nullptr;
-  size_t spare_bytes = 0;
   int *status_dev = nullptr;
   uint64_t *zero_poly = nullptr;  // [m][N]: import of a zero bit stream
   int *stop_flags = nullptr;      // SumLevelArgs::stop, kRedoFlags ints
@@ -139,33 +134,22 @@ inline cudaError_t clear_stop(xpir_b200_ctx *ctx) {
 struct xpir_b200_request;
 
 namespace xpir {
-// Gives the context's spare block back to the device (the caller holds ctx->mu).
-inline void drop_spare(xpir_b200_ctx *ctx) {
-  cudaFree(ctx->spare);
-  ctx->spare = nullptr;
-  ctx->spare_bytes = 0;
+// Spare memory: the polys of databases freed last, at most kSpareBytes per device and one block
+// by each context, for the next import of any context there (mapping and unmapping 655 MB
+// costs more than importing them).  Given back when the context that freed it is destroyed,
+// and by allocate and pool_allocate when an allocation on the device fails.  Nothing queued
+// anywhere uses a spare block.  Callable from any thread.
+bool take_spare(const xpir_b200_ctx *ctx, size_t bytes, void **ptr, size_t *have);
+void keep_spare(const xpir_b200_ctx *ctx, void *ptr, size_t bytes);  // or frees it
+void drop_spare(const xpir_b200_ctx *ctx);
+// cudaMalloc on `device` (the current one), and cudaMallocFromPoolAsync.
+cudaError_t allocate(int device, void **buf, size_t bytes);
+cudaError_t pool_allocate(int device, void **buf, size_t bytes, cudaMemPool_t pool, cudaStream_t stream);
+inline cudaError_t allocate(const xpir_b200_ctx *ctx, void **buf, size_t bytes) {
+  return allocate(ctx->device, buf, bytes);
 }
-
-// cudaMalloc that does so when memory is short.
-inline cudaError_t allocate(xpir_b200_ctx *ctx, void **buf, size_t bytes) {
-  cudaError_t e = cudaMalloc(buf, bytes);
-  if (e == cudaErrorMemoryAllocation && ctx->spare) {
-    (void)cudaGetLastError();
-    drop_spare(ctx);
-    e = cudaMalloc(buf, bytes);
-  }
-  return e;
-}
-
-// The same for the context's stream-ordered pool.
-inline cudaError_t pool_allocate(xpir_b200_ctx *ctx, void **buf, size_t bytes) {
-  cudaError_t e = cudaMallocFromPoolAsync(buf, bytes, ctx->pool, ctx->stream);
-  if (e == cudaErrorMemoryAllocation && ctx->spare) {
-    (void)cudaGetLastError();
-    drop_spare(ctx);
-    e = cudaMallocFromPoolAsync(buf, bytes, ctx->pool, ctx->stream);
-  }
-  return e;
+inline cudaError_t pool_allocate(const xpir_b200_ctx *ctx, void **buf, size_t bytes) {
+  return pool_allocate(ctx->device, buf, bytes, ctx->pool, ctx->stream);
 }
 
 // Whether two address ranges share a byte.

@@ -107,8 +107,9 @@ void upload_batch(xpir_b200_server *srv, uint32_t lane, std::vector<xpir::Job *>
   cudaError_t e = cudaSetDevice(ctx->device);
   for (size_t i = 0; i < batch.size(); i++) {
     auto *q = (ServedQuery *)batch[i]->payload.get();
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&q->dq, q->query_bytes ? q->query_bytes : 256, srv->pools[lane], cs);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&q->dr, q->reply_bytes ? q->reply_bytes : 256, srv->pools[lane], cs);
+    const uint64_t qb = q->query_bytes ? q->query_bytes : 256, rb = q->reply_bytes ? q->reply_bytes : 256;
+    if (e == cudaSuccess) e = xpir::pool_allocate(ctx->device, &q->dq, qb, srv->pools[lane], cs);
+    if (e == cudaSuccess) e = xpir::pool_allocate(ctx->device, &q->dr, rb, srv->pools[lane], cs);
     if (e != cudaSuccess) continue;
     const void *mapped = q->query_bytes >= kPullBytes ? mapped_device_address(q->host_query, ctx->device) : nullptr;
     if (mapped && (((uintptr_t)mapped | (uintptr_t)q->dq | q->query_bytes) & 15) == 0) {
@@ -143,7 +144,7 @@ void compute_batch(xpir_b200_server *srv, uint32_t lane, std::vector<xpir::Job *
   std::vector<void *> held;
   auto alloc = [&](size_t bytes, void **p) -> cudaError_t {
     *p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes ? bytes : 256, pool, st);
+    const cudaError_t e = xpir::pool_allocate(ctx->device, p, bytes ? bytes : 256, pool, st);
     if (e == cudaSuccess) held.push_back(*p);
     return e;
   };
