@@ -203,7 +203,10 @@ bool in_place(const std::vector<Group> &groups, const xpir_b200_request *reqs, u
   for (const Group &g : groups) {
     uint64_t total_ct = 0;
     for (uint32_t lvl = 0; lvl < g.d; lvl++) total_ct += g.n[lvl];
-    for (uint32_t i : g.reqs) queries.push_back({(uintptr_t)reqs[i].query, (uintptr_t)reqs[i].query + total_ct * ct_bytes});
+    for (uint32_t i : g.reqs) {
+      const uintptr_t from = (uintptr_t)reqs[i].query;
+      queries.push_back({from, from + total_ct * ct_bytes});
+    }
   }
   std::sort(queries.begin(), queries.end(), [](const Range &a, const Range &b) { return a.from < b.from; });
   for (size_t i = 1; i < queries.size(); i++) queries[i].to = std::max(queries[i].to, queries[i - 1].to);

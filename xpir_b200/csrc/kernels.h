@@ -29,8 +29,11 @@ struct AggSource {
   int *zero_hint = nullptr;
 };
 
-// Fewer all-zero polys do not keep the residue sums from deciding a chain, wherever they are:
-// seven in a row raise a run's bound by less than 1.0 p, and of the tail's slots five are left.
+// All-zero polys, counted over the whole database, from which its replies go slot by slot.
+// Fewer do not keep the residue sums from deciding a chain, wherever they are: seven in a row
+// raise a run's bound by less than 1.1 p, and of the tail's slots five are left.  More may or
+// may not: a hundred in a row of one column, or sixty up to its end, do; scattered ones, up to
+// three in ten at least, hardly ever.  One count for the database cannot tell these apart.
 constexpr int kZeroPolys = 8;
 
 // Per-modulus constants the device needs, by value.

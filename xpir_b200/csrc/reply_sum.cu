@@ -21,7 +21,7 @@
 // warp scheduler and the additions around it hardly overlap with it: a word and half cost
 // four of those and about twelve other instructions (32 cycles), where the slot-by-slot
 // kernel spends 56 on a Shoup factor and a Shoup product alone.  1,048,576 x 256 B in 16s:
-// level 1 2.47 -> 1.45 ms.  Up to four columns per CTA share the query words' preparation.
+// level 1 2.47 -> 1.57 ms.  Up to four columns per CTA share the query words' preparation.
 //
 // What the sums cannot decide sets the query's redo flag, and the caller repeats that query
 // slot by slot.  A CTA that finds such a word stops at once, and the query's other CTAs that
