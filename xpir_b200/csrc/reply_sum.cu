@@ -40,6 +40,7 @@
 namespace xpir {
 namespace {
 
+constexpr uint32_t kAllTiles = ~0u;
 constexpr uint32_t kTopOfP = 0x1fffffffu;  // p >> 32 of every modulus
 
 // A kernel parameter: kept small (16 bytes more took the 1,000 x 12 KB reply from 38.7 to 39.2 us).
@@ -58,8 +59,8 @@ struct SumShape {
   int *status;        // the redo flags follow it
   int *stop;          // device copies of those: a query's CTAs that see its flag set do no more work
   uint32_t first;     // task 0's place among the flags
-  uint32_t spin_limit;   // polls of a wait
-  uint32_t issued_tiles; // tiles the producer issues at most (test support: it starves the consumers)
+  uint32_t spin_limit;    // polls of a wait (read with TEST only, as the next)
+  uint32_t issued_tiles;  // tiles the producer issues at most (kAllTiles: all)
 };
 
 __host__ __device__ __forceinline__ uint32_t flag_of(uint32_t first, uint32_t task) {
@@ -81,10 +82,8 @@ struct SumCfg {
   static_assert(E % 4 == 0 && W % 32 == 0 && W <= 256, "tile shape");
 };
 
-// Waits for a phase; false after `limit` polls or when the CTA has given up.  Not inlined: with
-// the limit a variable, the loop beside the products cost 1 % (1,048,576 x 256 B 1,807 us; as a
-// call 1,793, with the limit a constant 1,792).
-__device__ __noinline__ bool wait_or_quit(uint64_t *bar, uint32_t parity, volatile CtaState *state, uint32_t limit) {
+// Waits for a phase; false after `limit` polls or when the CTA has given up.
+__device__ __forceinline__ bool wait_or_quit(uint64_t *bar, uint32_t parity, volatile CtaState *state, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if (state->quit) return false;
@@ -114,7 +113,11 @@ __device__ __noinline__ bool chain_again(const ReplyTask &task, const SumShape &
   return s.above == 0 && (!from || tail_in_range(s, kMaxAbove));
 }
 
-template <int W, int C, int E, int NS, bool ONE>
+// TEST: with the wait test's limit and withheld tile (xpir_b200_ctx_set_wait_test), in kernels of
+// their own: as variables of the one kernel they cost it up to 1.6 % (a batch of three queries,
+// 131 x 139 slots, 17,862 x 717 B: 699 us, without them 688; 65,536 x 8 KB, 256 x 256 slots from
+// host memory: 1,023 and 1,016).
+template <int W, int C, int E, int NS, bool ONE, bool TEST>
 __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t task_id, const uint32_t slice,
                                          const uint32_t cb, const uint32_t run, const SumShape &sh,
                                          const DevModuli &dm) {
@@ -135,6 +138,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
   const uint32_t end = ONE ? sh.n_eff : sum_end;
   const uint32_t tiles = (end - s0 + E - 1) / E;
 
+  const uint32_t limit = TEST ? sh.spin_limit : kSpinLimit;
   if constexpr (!ONE) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   if (threadIdx.x == 0) {
     state->quit = 0;
@@ -160,15 +164,16 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
         poly[i] = (int)(j - g * sh.P);
       }
       uint32_t t = 0, st = 0, phase = 1;
-      for (const uint32_t issued = min(tiles, sh.issued_tiles); t < issued; ++t) {
+      for (; t < tiles; ++t) {
         if (state->quit) break;
+        if (TEST && t == sh.issued_tiles) break;
         if (t % 64 == (uint32_t)NS && *(volatile int *)(sh.stop + state->flag)) {
           state->quit = 1;
           *(volatile int *)(sh.status + 1 + state->flag) = 1;  // also after a call that failed before it cleared the flag
           __threadfence_system();
           break;
         }
-        if (t >= (uint32_t)NS && !wait_or_quit(empty + st, phase, state, sh.spin_limit)) break;
+        if (t >= (uint32_t)NS && !wait_or_quit(empty + st, phase, state, limit)) break;
         mbar_arrive_expect_tx(full + st, (uint32_t)((S::kX + S::kQ) * 8));
         const int slot = (int)(s0 + t * E);
 #pragma unroll
@@ -200,7 +205,7 @@ __device__ __forceinline__ void sum_tile(const ReplyTask &task, const uint32_t t
   uint32_t t = 0, st = 0, phase = 0;
   // Waits for tile t; false (in the whole warp) when it must stop.
   auto tile_ready = [&]() -> bool {
-    const bool ok = mbar_try_wait(full + st, phase) || wait_or_quit(full + st, phase, state, sh.spin_limit);
+    const bool ok = mbar_try_wait(full + st, phase) || wait_or_quit(full + st, phase, state, limit);
     if (!__any_sync(~0u, bad || !ok)) return true;
     late = !__all_sync(~0u, ok);
     bad = __any_sync(~0u, bad);
@@ -341,13 +346,13 @@ __device__ __forceinline__ void decode_block(const SumShape &sh, uint32_t *slice
 }
 
 // One query: its task by value (tasks null).  Several: a table in global memory.
-template <int W, int C, int E, int NS, bool ONE, int MINB>
+template <int W, int C, int E, int NS, bool ONE, int MINB, bool TEST>
 __global__ void __launch_bounds__(SumCfg<W, C, E, NS>::kThreads, MINB)
     reply_sum_kernel(const __grid_constant__ ReplyTask one, const ReplyTask *__restrict__ tasks, const SumShape sh,
                      const DevModuli dm) {
   uint32_t slice, tk, cb, run;
   decode_block(sh, &slice, &tk, &cb, &run);
-  sum_tile<W, C, E, NS, ONE>(tasks ? tasks[tk] : one, tk, slice, cb, run, sh, dm);
+  sum_tile<W, C, E, NS, ONE, TEST>(tasks ? tasks[tk] : one, tk, slice, cb, run, sh, dm);
 }
 
 // Adds the runs' residues of one column's kFinishCoefs coefficients and runs the exact
@@ -450,7 +455,12 @@ cudaError_t launch_sum(const ReplyTask &one, const ReplyTask *dev, const SumShap
   using S = SumCfg<W, C, E, NS>;
   const uint64_t blocks = (uint64_t)sh.slices * sh.ntasks * sh.col_blocks * sh.runs;
   if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-  auto kern = reply_sum_kernel<W, C, E, NS, ONE, MINB>;
+  auto kern = reply_sum_kernel<W, C, E, NS, ONE, MINB, false>;
+  if (sh.spin_limit != kSpinLimit || sh.issued_tiles != kAllTiles) {  // loaded when first asked for
+    kern = reply_sum_kernel<W, C, E, NS, ONE, MINB, true>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kBytes);
+    if (e != cudaSuccess) return e;
+  }
   kern<<<(unsigned)blocks, S::kThreads, S::kBytes, stream>>>(one, dev, sh, dm);
   return cudaGetLastError();
 }
@@ -459,8 +469,8 @@ cudaError_t launch_sum(const ReplyTask &one, const ReplyTask *dev, const SumShap
   {                                                                                                 \
     W, C, E, NS, MINB, &launch_sum<W, C, E, NS, true, MINB>, &launch_sum<W, C, E, NS, false, MINB>, \
     {                                                                                               \
-      (const void *)reply_sum_kernel<W, C, E, NS, true, MINB>,                                      \
-          (const void *)reply_sum_kernel<W, C, E, NS, false, MINB>                                  \
+      (const void *)reply_sum_kernel<W, C, E, NS, true, MINB, false>,                               \
+          (const void *)reply_sum_kernel<W, C, E, NS, false, MINB, false>                           \
     }, SumCfg<W, C, E, NS>::kBytes                                                                  \
   }
 
@@ -561,7 +571,7 @@ cudaError_t launch_sum_level(const SumLevelArgs &a, const uint64_t *const *db, c
   sh.stop = a.stop;
   sh.first = a.first;
   sh.spin_limit = a.wait_test.spin_limit ? a.wait_test.spin_limit : kSpinLimit;
-  sh.issued_tiles = (uint32_t)a.wait_test.withhold_tile;  // -1: all
+  sh.issued_tiles = a.wait_test.withhold_tile < 0 ? kAllTiles : (uint32_t)a.wait_test.withhold_tile;
   // Elements past n_live (idle): the group that holds the first of them is a launch of its
   // own when there are others, since its chain ends at another slot.
   const bool idle = a.n_live < a.n_real;
